@@ -132,6 +132,7 @@ struct SphHandle {
   // scalars
   float *dt = nullptr, *dt_query = nullptr, *red = nullptr;
   uint32_t* err = nullptr;
+  uint32_t* slow = nullptr;  // per instance: its pair sums take the general operations (k_xsph_prep, k_density)
   // metrics
   int nparts = 0;
   double *part_m = nullptr, *part_e = nullptr, *me = nullptr;
@@ -281,6 +282,23 @@ SimConst make_const(const SphParams& p, const uint32_t dims[3]) {
   k.sup_d2 = sqrt_below(k.support);
   k.r0_d2 = sqrt_below(k.r0);
   k.tiny_d2 = sqrt_at_most(1.0e-12f);
+  // The pair sums' fast quotients (sph::div_rn). d2 + eta^2 stays between
+  // 2^-60 and 1, so a nonzero dividend gives a nonzero mu; the viscous
+  // dividend h v.r = mu (r^2 + eta^2) is at least 2^-98 and the dividend
+  // alpha c mu + beta mu^2 at least 2^-80 (a normal quotient by any density
+  // sum up to 2 kRhoMax) for every |mu| from mu_min on. Negative or
+  // non-finite coefficients could cancel: those take the general operations.
+  k.neg_alpha_c2 = 2.0f * k.neg_alpha_c;
+  k.beta2 = 2.0f * k.beta;
+  const double ac = -(double)k.neg_alpha_c, be = (double)k.beta;
+  k.fast = h >= 0x1p-24f && h <= 0.45f && ac >= 0.0 && ac <= 0x1p60 && be >= 0.0 && be <= 0x1p60;
+  double by_num = 0.0;
+  if (ac > 0.0) by_num = 0x1p-80 / ac;
+  if (be > 0.0) by_num = ac > 0.0 ? std::min(by_num, std::sqrt(0x1p-80 / be)) : std::sqrt(0x1p-80 / be);
+  const float mu_min = (float)std::min(1e30, std::max(0x1p-98 / (double)k.eta_sq, by_num));
+  uint32_t mu_bits;
+  std::memcpy(&mu_bits, &mu_min, sizeof mu_bits);
+  k.mu_key = sph::mag_key(mu_bits);
   return k;
 }
 
@@ -570,7 +588,7 @@ void build_boundary_lists(const SimConst& k, const SphBoundaryView* b, int C,
 // particle slot, or by boundary particle when `boundary`).
 template <class F>
 void dispatch(SphHandle* h, bool boundary, F&& f) {
-  if (h->ninst == 1) f(sph::OneSim{h->k});
+  if (h->ninst == 1) f(sph::OneSim{h->k, h->ktab});
   else f(sph::ManySim{h->ktab, boundary ? h->inst_b : h->inst_p});
 }
 
@@ -636,17 +654,17 @@ void enqueue_density_only(SphHandle* h) {
       k_density<KPT, 2><<<grid, bs, smem_cl, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
                                                      h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
                                                      h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
-                                                  warp_scan);
+                                                  warp_scan, h->slow);
     else if (h->cl_mode)
       k_density<KPT, 1><<<grid, bs, smem, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
                                                   h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
                                                   h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
-                                                  warp_scan);
+                                                  warp_scan, h->slow);
     else
       k_density<KPT, 0><<<grid, bs, smem, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
                                                   h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
                                                   h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
-                                                  warp_scan);
+                                                  warp_scan, h->slow);
   });
   h->launches += 1;
 }
@@ -684,18 +702,14 @@ void enqueue_forces(SphHandle* h, float hdt_scale) {
   int bs = h->bs_forces;
   dispatch(h, false, [&](auto kp) {
     using KPT = decltype(kp);
-    if (h->cl_mode)
-      k_forces<KPT, 1><<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, hdt_scale, h->pos, h->vel, h->rf,
-                                                           h->pr, h->id, h->ctab, h->bc_start, h->bc_list,
-                                                           h->bpos, h->bpress, h->acc, h->velout, h->red,
-                                                           h->err, h->nbr, h->ncount, h->sdf, h->wall_tab,
-                                                           h->corr);
-    else
-      k_forces<KPT, 0><<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, hdt_scale, h->pos, h->vel, h->rf,
-                                                           h->pr, h->id, h->ctab, h->bc_start, h->bc_list,
-                                                           h->bpos, h->bpress, h->acc, h->velout, h->red,
-                                                           h->err, h->nbr, h->ncount, h->sdf, h->wall_tab,
-                                                           h->corr);
+    auto launch = [&](auto kernel) {
+      kernel<<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, hdt_scale, h->pos, h->vel, h->rf, h->pr, h->id,
+                                                  h->ctab, h->bc_start, h->bc_list, h->bpos, h->bpress, h->acc,
+                                                  h->velout, h->red, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab,
+                                                  h->corr, h->slow);
+    };
+    if (h->cl_mode) launch(k_forces<KPT, 1>);
+    else launch(k_forces<KPT, 0>);
   });
   h->launches += 1;
 }
@@ -705,11 +719,11 @@ void enqueue_xsph(SphHandle* h, bool use_list) {
   int bs = h->bs_xsph;
   dispatch(h, false, [&](auto kp) {
     k_xsph_prep<<<grid_for(h->n, 256), 256, 0, h->st>>>(kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec,
-                                                         h->err);
+                                                         h->err, h->slow);
     k_xsph_drift<<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec, h->id,
-                                                       h->ctab, h->rank_of_lin, h->posU, h->velU, h->idU,
-                                                       h->keyU, h->hist, h->err,
-                                                       use_list ? h->nbr : nullptr, h->ncount);
+                                                         h->ctab, h->rank_of_lin, h->posU, h->velU, h->idU,
+                                                         h->keyU, h->hist, h->err, use_list ? h->nbr : nullptr,
+                                                         h->ncount, h->slow);
   });
   h->launches += 2;
 }
@@ -974,8 +988,9 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     ALLOC(nbr, (size_t)sph::kNbrCap * n); ALLOC(ncount, n); ALLOC(xrec, 2 * n);
     h->xyz_stride = ((size_t)n + 3) / 4 * 4 + 4;  // aligned groups of 4 may read past the last slot
     ALLOC(xyz, 3 * h->xyz_stride);
+    ALLOC(ktab, ninst); ALLOC(slow, ninst);
     if (ninst > 1) {
-      ALLOC(ktab, ninst); ALLOC(inst_p, n); ALLOC(inst_b, nb);
+      ALLOC(inst_p, n); ALLOC(inst_b, nb);
     }
     if (sdf_mode) ALLOC(sdf, std::max<uint64_t>(sdf_nodes, 1));
 #undef ALLOC
@@ -1265,7 +1280,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   up(h->bc_cells, bcells.data(), bcells.size() * sizeof(uint32_t));
   if (h->adami_cells) up(h->border, border_h.data(), nb * sizeof(uint32_t));
   up(h->hcc, hcc.data(), ninst * sizeof(float4));
-  if (ninst > 1) up(h->ktab, h->ktab_h.data(), ninst * sizeof(SimConst));
+  up(h->ktab, h->ktab_h.data(), ninst * sizeof(SimConst));
   for (int q = 0; sdf_mode && q < ninst; ++q)
     if (sdf_off[q + 1] > sdf_off[q])
       up(h->sdf + sdf_off[q], sdfs[q].distances, (sdf_off[q + 1] - sdf_off[q]) * sizeof(float));
@@ -1274,6 +1289,9 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   if (e == cudaSuccess) e = cudaMemsetAsync(h->hist, 0, C * sizeof(uint32_t), h->st);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->bpress, 0, std::max<size_t>(1, nb) * sizeof(float), h->st);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->err, 0, sizeof(uint32_t), h->st);
+  std::vector<uint32_t> slow(ninst);
+  for (int q = 0; q < ninst; ++q) slow[q] = h->ktab_h[q].fast ? 0u : 1u;
+  up(h->slow, slow.data(), ninst * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemsetAsync(h->ctab, 0, C * sizeof(uint2), h->st);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->xyz, 0, 3 * h->xyz_stride * sizeof(float), h->st);
   if (e == cudaSuccess && n > 0) {
@@ -2194,7 +2212,7 @@ int sph_interpolate(SphHandle* h, const float* pts, size_t npts, float* out) {
   if (e == cudaSuccess) e = cudaMalloc((void**)&dout, npts * 7 * sizeof(float));
   if (e == cudaSuccess) e = cudaMemcpyAsync(dp, p4.data(), npts * sizeof(float4), cudaMemcpyHostToDevice, h->st);
   if (e == cudaSuccess) {
-    sph::k_interpolate<<<grid_for((long long)npts, 128), 128, 0, h->st>>>(sph::OneSim{h->k}, (int)npts, dp, h->pos,
+    sph::k_interpolate<<<grid_for((long long)npts, 128), 128, 0, h->st>>>(sph::OneSim{h->k, h->ktab}, (int)npts, dp, h->pos,
                                                                           h->rf, h->pr, h->acc, h->ctab, dout);
     h->launches += 1;
     e = cudaMemcpyAsync(out, dout, npts * 7 * sizeof(float), cudaMemcpyDeviceToHost, h->st);
