@@ -4,7 +4,6 @@
 // buffers and CUDA graphs. The step body (9 kernels) is captured once into a
 // graph and replayed; dt lives in device memory so the graph never changes.
 #include <algorithm>
-#include <array>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -104,20 +103,15 @@ struct SphHandle {
   // boundary
   float4* bpos = nullptr;
   float* bpress = nullptr;
-  uint8_t* bact = nullptr;  // per boundary particle: an occupied cell lists it (k_adami_mark)
-  uint32_t* bc_cells = nullptr;  // the linear cells whose boundary candidate list is not empty
-  int nbc_cells = 0;
-  // the boundary particles sorted by the (global) cell that holds them, for
-  // k_adami_cells; used when every instance is in the row or linear order
-  uint32_t* border = nullptr;
-  bool adami_cells = false;
+  // per boundary particle: the fluid particles in its support (k_wall_scatter;
+  // wlist null where its memory could not be had: k_adami then searches)
+  uint32_t *wcount = nullptr, *wlist = nullptr;
   int pool = -1;  // device arrays from the library's pool (1) or cudaMalloc (0); set by the first one
-  // Below these sizes the per-particle forms of the density scan and of the
-  // boundary pressure run instead of the warp-cooperative ones: a warp per 32
-  // particles (or boundary particles) then leaves the SMs too few warps to
-  // hide the longer per-warp chains. Set at creation from the SM count.
+  // Below this size the per-particle form of the density scan runs instead of
+  // the warp-cooperative one: a warp per 32 particles then leaves the SMs too
+  // few warps to hide the longer per-warp chains. Set at creation from the SM
+  // count.
   int warp_scan_min = 0;
-  size_t adami_cells_min = 0;
   uint32_t *bc_start = nullptr, *bc_list = nullptr;
   // SDF node grid and wall table (boundary_mode SPH_BOUNDARY_SDF), or the
   // geometry SDF(s) of the closure features
@@ -594,18 +588,12 @@ void dispatch(SphHandle* h, bool boundary, F&& f) {
 
 sph::Planes planes(SphHandle* h) { return sph::Planes{h->xyz, h->xyz_stride}; }
 
-// Sizes per SM from which the warp-cooperative density scan (particles) and
-// the cell-wise boundary pressure (boundary particles) run, measured on B200.
-// Below them the per-particle forms are faster (2M-particle dam break and its
-// coarser versions: the density scans break even near 250k particles, the
-// boundary passes between 376k and 848k boundary particles). The environment
-// variables SPH_WARP_SCAN_MIN and SPH_ADAMI_CELLS_MIN, read at creation,
-// replace them with absolute counts (0: always the warp-cooperative form).
+// Particles per SM from which the warp-cooperative density scan runs, measured
+// on B200 (dam break at five resolutions: the two forms break even near 250k
+// particles). The environment variable SPH_WARP_SCAN_MIN, read at creation,
+// replaces it with an absolute count (0: always the warp-cooperative form).
 #ifndef SPH_WARP_SCAN_MIN_PER_SM
 #define SPH_WARP_SCAN_MIN_PER_SM 2048
-#endif
-#ifndef SPH_ADAMI_CELLS_MIN_PER_SM
-#define SPH_ADAMI_CELLS_MIN_PER_SM 4096
 #endif
 
 // Lets the density kernels take up to 128 KiB of dynamic shared memory (the
@@ -669,26 +657,24 @@ void enqueue_density_only(SphHandle* h) {
   h->launches += 1;
 }
 
-// boundary.rs:87-123: the Adami boundary pressure, for the boundary particles
-// that an occupied cell lists (the others get the empty sum's 0)
+// boundary.rs:87-123: the Adami boundary pressure (a boundary particle without
+// fluid in support gets the empty sum's 0)
 void enqueue_adami(SphHandle* h) {
   using namespace sph;
-  if (h->nb > 0) {
-    cudaMemsetAsync(h->bact, 0, (size_t)h->nb, h->st);
-    if (h->nbc_cells > 0)
-      k_adami_mark<<<grid_for(h->nbc_cells, 8), 256, 0, h->st>>>(h->nbc_cells, h->bc_cells, h->ctab, h->bc_start,
-                                                                  h->bc_list, h->bact);
-    dispatch(h, true, [&](auto kp) {
-      if (h->adami_cells && (size_t)h->nb >= h->adami_cells_min)
-        k_adami_cells<<<grid_for(h->nb, kAdamiWarps * 32), kAdamiWarps * 32, 0, h->st>>>(
-            kp, h->nb, h->border, h->bpos, h->bpress, h->pos, planes(h), h->rf, h->pr, h->id, h->ctab, h->err,
-            h->bact);
-      else
-        k_adami<<<grid_for(h->nb, kAdamiWarps), kAdamiWarps * 32, 0, h->st>>>(
-            kp, h->nb, h->bpos, h->bpress, h->pos, h->rf, h->pr, h->id, h->ctab, h->err, h->bact);
+  if (h->nb == 0) return;
+  if (h->wlist) {
+    const int P = h->n >= 1000000 ? 16 : 8;  // between 250k and 2M particles the two cross (k_wall_scatter)
+    dispatch(h, false, [&](auto kp) {
+      k_wall_scatter<<<grid_for(h->n, 8 * P), 256, 0, h->st>>>(kp, h->n, P, h->pos, h->nbr, h->ncount, h->bc_start,
+                                                               h->bc_list, h->bpos, h->wcount, h->wlist, h->err);
     });
-    h->launches += 2;
+    h->launches += 1;
   }
+  dispatch(h, true, [&](auto kp) {
+    k_adami<<<grid_for(h->nb, kAdamiWarps * 4), kAdamiWarps * 32, 0, h->st>>>(
+        kp, h->nb, h->bpos, h->bpress, h->pos, h->rf, h->pr, h->id, h->ctab, h->err, h->wcount, h->wlist);
+  });
+  h->launches += 1;
 }
 
 void enqueue_density_adami(SphHandle* h) {
@@ -970,9 +956,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     int sms = 148;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess) sms = 148;
     h->warp_scan_min = sms * SPH_WARP_SCAN_MIN_PER_SM;
-    h->adami_cells_min = (size_t)sms * SPH_ADAMI_CELLS_MIN_PER_SM;
     if (const char* v = std::getenv("SPH_WARP_SCAN_MIN")) h->warp_scan_min = std::atoi(v);
-    if (const char* v = std::getenv("SPH_ADAMI_CELLS_MIN")) h->adami_cells_min = (size_t)std::atoll(v);
 #define ALLOC(ptr, cnt) \
   if (ae == cudaSuccess) ae = dalloc(h, &h->ptr, (cnt))
     ALLOC(pos, n); ALLOC(vel, n); ALLOC(velout, n); ALLOC(acc, n);
@@ -980,7 +964,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     ALLOC(posU, n); ALLOC(velU, n); ALLOC(idU, n); ALLOC(keyU, n); ALLOC(tmp, n); ALLOC(tmpid, n);
     ALLOC(hist, C); ALLOC(cstart, C); ALLOC(ccount, C); ALLOC(cursor, C); ALLOC(bsum, h->nbsum);
     ALLOC(rank_of_lin, C); ALLOC(lin_of_rank, C); ALLOC(ctab, C);
-    ALLOC(bpos, nb); ALLOC(bpress, nb); ALLOC(bact, nb); ALLOC(bc_start, C + 1);
+    ALLOC(bpos, nb); ALLOC(bpress, nb); ALLOC(wcount, nb); ALLOC(bc_start, C + 1);
     ALLOC(dt, ninst); ALLOC(dt_query, ninst); ALLOC(red, 2 * ninst); ALLOC(err, 1); ALLOC(hcc, ninst);
     ALLOC(part_m, h->nparts); ALLOC(part_e, h->nparts); ALLOC(part_var, h->nparts); ALLOC(me, 2);
     ALLOC(var, 1); ALLOC(bad, 1);
@@ -1095,56 +1079,6 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
       h->init_e[q] = e;
     }
   };
-  // The boundary particles ordered by the global cell that holds them
-  // (counting sort, ascending index within a cell), for k_adami_cells; the
-  // cells are those of the grid built below (same f32 operations), on a
-  // thread of its own while this one builds the tables.
-  std::vector<uint32_t> border_h;
-  h->adami_cells = nb > 0;
-  for (int q = 0; q < ninst; ++q)
-    h->adami_cells = h->adami_cells &&
-                     (PP[q].cell_order == SPH_CELL_ORDER_LINEAR || PP[q].cell_order == SPH_CELL_ORDER_ROWS);
-  auto boundary_order = [&] {
-    uint64_t Ctot = 0;
-    std::vector<uint64_t> coffs(ninst);
-    std::vector<std::array<uint32_t, 3>> dimq(ninst);
-    for (int q = 0; q < ninst; ++q) {
-      const float cell = 2.0f * PP[q].h;
-      uint64_t Cq = 1;
-      for (int a = 0; a < 3; ++a) {
-        dimq[q][a] = (uint32_t)fmaxf(ceilf((PP[q].domain_max[a] - PP[q].domain_min[a]) / cell), 1.0f);
-        Cq *= dimq[q][a];
-      }
-      coffs[q] = Ctot;
-      Ctot += Cq;
-    }
-    std::vector<uint32_t> bkey(nb), bnext(Ctot + 1, 0);
-    for (int q = 0; q < ninst; ++q) {
-      const float cell = 2.0f * PP[q].h;
-      auto cell_of = [&](float p, int a) {  // axis_cell, in the same f32 operations
-        float f = std::floor((p - PP[q].domain_min[a]) / cell);
-        f = std::fmax(f, 0.0f);
-        f = std::fmin(f, (float)(dimq[q][a] - 1));
-        return (uint32_t)f;
-      };
-      for (size_t i = h->boff[q]; i < h->boff[q + 1]; ++i) {
-        const float4 v = hb[i];
-        bkey[i] = (uint32_t)coffs[q] + cell_of(v.x, 0) + dimq[q][0] * (cell_of(v.y, 1) + dimq[q][1] * cell_of(v.z, 2));
-        ++bnext[bkey[i] + 1];
-      }
-    }
-    for (uint64_t c = 0; c < Ctot; ++c) bnext[c + 1] += bnext[c];
-    border_h.resize(nb);
-    for (size_t i = 0; i < nb; ++i) border_h[bnext[bkey[i]]++] = (uint32_t)i;
-  };
-  std::thread border_thread;
-  if (h->adami_cells) {
-    try {
-      border_thread = std::thread(boundary_order);
-    } catch (...) {  // no thread to be had: order them here
-      boundary_order();
-    }
-  }
   std::thread totals;
   try {
     totals = std::thread(initial_totals);
@@ -1232,14 +1166,9 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   }
   if (totals.joinable()) totals.join();
   trace.mark("cell ranks, lists, totals");
-  if (border_thread.joinable()) border_thread.join();
-  trace.mark("boundary order");
   h->k = h->ktab_h[0];
   h->C = (int)C;
   h->boundary_candidates = blist.size();
-  std::vector<uint32_t> bcells;  // cells with boundary candidates (static: they bound k_adami_mark)
-  for (uint64_t c = 0; c < C; ++c)
-    if (bstart[c + 1] > bstart[c]) bcells.push_back((uint32_t)c);
   for (int q = 0; q < ninst; ++q) {
     h->init_mass += h->init_m[q];
     h->init_energy += h->init_e[q];
@@ -1261,9 +1190,10 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   trace.mark("particle uploads joined");
   if (e == cudaSuccess) e = ue;
   if (e == cudaSuccess) e = dalloc(h, &h->bc_list, blist.size());
-  if (e == cudaSuccess) e = dalloc(h, &h->bc_cells, bcells.size());
-  if (e == cudaSuccess && h->adami_cells) e = dalloc(h, &h->border, nb);
-  h->nbc_cells = (int)bcells.size();
+  if (e == cudaSuccess && nb > 0 && dalloc(h, &h->wlist, sph::kWallCap * nb) != cudaSuccess) {
+    cudaGetLastError();
+    h->wlist = nullptr;  // k_adami searches instead
+  }
   if (e == cudaSuccess && sdf_mode) e = dalloc(h, &h->wall_tab, wall_host.size());
   if (e != cudaSuccess) {
     cudaFree(accU);
@@ -1277,8 +1207,6 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   up(h->lin_of_rank, lin_of_rank.data(), C * sizeof(uint32_t));
   up(h->bc_start, bstart.data(), (C + 1) * sizeof(uint32_t));
   up(h->bc_list, blist.data(), blist.size() * sizeof(uint32_t));
-  up(h->bc_cells, bcells.data(), bcells.size() * sizeof(uint32_t));
-  if (h->adami_cells) up(h->border, border_h.data(), nb * sizeof(uint32_t));
   up(h->hcc, hcc.data(), ninst * sizeof(float4));
   up(h->ktab, h->ktab_h.data(), ninst * sizeof(SimConst));
   for (int q = 0; sdf_mode && q < ninst; ++q)
@@ -1292,6 +1220,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   std::vector<uint32_t> slow(ninst);
   for (int q = 0; q < ninst; ++q) slow[q] = h->ktab_h[q].fast ? 0u : 1u;
   up(h->slow, slow.data(), ninst * sizeof(uint32_t));
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->wcount, 0, std::max<size_t>(1, nb) * sizeof(uint32_t), h->st);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->ctab, 0, C * sizeof(uint2), h->st);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->xyz, 0, 3 * h->xyz_stride * sizeof(float), h->st);
   if (e == cudaSuccess && n > 0) {
