@@ -110,8 +110,10 @@ def test_operands_outside_the_fast_range(change, coef, order):
     gpu.close()
 
 
-def test_large_smoothing_length():
-    sc = domain.dam_break(0.5, seed=2, block=(4.0, 3.0, 3.0), domain_max=(6.0, 3.0, 3.0), with_sdf=False)
+@pytest.mark.parametrize("scale", [0.5, 500.0])
+def test_large_smoothing_length(scale):
+    sc = domain.dam_break(scale, seed=2, block=(8 * scale, 6 * scale, 6 * scale),
+                          domain_max=(12 * scale, 6 * scale, 6 * scale), with_sdf=False)
     gpu = CudaKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta)
     cpu = orc.OracleKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta, tier=1, threads=8, pow_mode=1)
     for _ in range(3):

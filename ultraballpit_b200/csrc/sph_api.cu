@@ -15,11 +15,13 @@
 #include <new>
 #include <string>
 #include <thread>
+#include <type_traits>
 #include <vector>
 
 #include <cuda_bf16.h>
 
 #include "sph_cuda.h"
+#include "sph_group.cuh"
 #include "sph_kernels.cuh"
 
 using sph::SimConst;
@@ -107,11 +109,9 @@ struct SphHandle {
   // wlist null where its memory could not be had: k_adami then searches)
   uint32_t *wcount = nullptr, *wlist = nullptr;
   int pool = -1;  // device arrays from the library's pool (1) or cudaMalloc (0); set by the first one
-  // Below this size the per-particle form of the density scan runs instead of
-  // the warp-cooperative one: a warp per 32 particles then leaves the SMs too
-  // few warps to hide the longer per-warp chains. Set at creation from the SM
-  // count.
-  int warp_scan_min = 0;
+  // lanes per particle of the neighbour kernels (1: a thread per particle, in
+  // density the warp-cooperative scan); set at creation from the size
+  int lanes_xsph = 1, lanes_density = 1, lanes_forces = 1;
   uint32_t *bc_start = nullptr, *bc_list = nullptr;
   // SDF node grid and wall table (boundary_mode SPH_BOUNDARY_SDF), or the
   // geometry SDF(s) of the closure features
@@ -276,23 +276,27 @@ SimConst make_const(const SphParams& p, const uint32_t dims[3]) {
   k.sup_d2 = sqrt_below(k.support);
   k.r0_d2 = sqrt_below(k.r0);
   k.tiny_d2 = sqrt_at_most(1.0e-12f);
-  // The pair sums' fast quotients (sph::div_rn). d2 + eta^2 stays between
-  // 2^-60 and 1, so a nonzero dividend gives a nonzero mu; the viscous
-  // dividend h v.r = mu (r^2 + eta^2) is at least 2^-98 and the dividend
-  // alpha c mu + beta mu^2 at least 2^-80 (a normal quotient by any density
-  // sum up to 2 kRhoMax) for every |mu| from mu_min on. Negative or
+  // The pair sums' fast quotients (sph::div_rn): every divisor d2 + eta^2 is at
+  // most b, so a dividend of 2^-98 max(b, 1) has a normal quotient and exact
+  // residuals, and a viscous dividend of mu_min b a |mu| of at least mu_min,
+  // from which on the second dividend alpha c |mu| + beta mu^2 is at least
+  // 2^-94 (a normal quotient by any density sum up to 2 kRhoMax). Negative or
   // non-finite coefficients could cancel: those take the general operations.
   k.neg_alpha_c2 = 2.0f * k.neg_alpha_c;
   k.beta2 = 2.0f * k.beta;
-  const double ac = -(double)k.neg_alpha_c, be = (double)k.beta;
-  k.fast = h >= 0x1p-24f && h <= 0.45f && ac >= 0.0 && ac <= 0x1p60 && be >= 0.0 && be <= 0x1p60;
-  double by_num = 0.0;
-  if (ac > 0.0) by_num = 0x1p-80 / ac;
-  if (be > 0.0) by_num = ac > 0.0 ? std::min(by_num, std::sqrt(0x1p-80 / be)) : std::sqrt(0x1p-80 / be);
-  const float mu_min = (float)std::min(1e30, std::max(0x1p-98 / (double)k.eta_sq, by_num));
-  uint32_t mu_bits;
-  std::memcpy(&mu_bits, &mu_min, sizeof mu_bits);
-  k.mu_key = sph::mag_key(mu_bits);
+  const double ac = -(double)k.neg_alpha_c, be = (double)k.beta, b = 4.1 * (double)h * h;
+  k.fast = h >= 0x1p-24f && h <= 0x1p20f && ac >= 0.0 && ac <= 0x1p60 && be >= 0.0 && be <= 0x1p60;
+  double mu_min = 0.0;
+  if (ac > 0.0) mu_min = 0x1p-94 / ac;
+  if (be > 0.0) mu_min = ac > 0.0 ? std::min(mu_min, std::sqrt(0x1p-94 / be)) : std::sqrt(0x1p-94 / be);
+  auto key_of = [](double v) {
+    const float f = (float)std::min(1e30, v);
+    uint32_t bits;
+    std::memcpy(&bits, &f, sizeof bits);
+    return sph::mag_key(bits);
+  };
+  k.diff_key = key_of(0x1p-98 * std::max(b, 1.0));
+  k.visc_key = key_of(std::max(0x1p-98 * std::max(b, 1.0), mu_min * b));
   return k;
 }
 
@@ -586,15 +590,32 @@ void dispatch(SphHandle* h, bool boundary, F&& f) {
   else f(sph::ManySim{h->ktab, boundary ? h->inst_b : h->inst_p});
 }
 
+// f(std::integral_constant<int, G>) for a supported group size
+template <class F>
+void with_lanes(int lanes, F&& f) {
+  if (lanes == 8) f(std::integral_constant<int, 8>());
+  else f(std::integral_constant<int, 16>());
+}
+
 sph::Planes planes(SphHandle* h) { return sph::Planes{h->xyz, h->xyz_stride}; }
 
-// Particles per SM from which the warp-cooperative density scan runs, measured
-// on B200 (dam break at five resolutions: the two forms break even near 250k
-// particles). The environment variable SPH_WARP_SCAN_MIN, read at creation,
-// replaces it with an absolute count (0: always the warp-cooperative form).
-#ifndef SPH_WARP_SCAN_MIN_PER_SM
-#define SPH_WARP_SCAN_MIN_PER_SM 2048
-#endif
+// Lanes per particle by size, measured on B200 (the table in sph_group.cuh).
+// The environment variable SPH_WARP_SCAN_MIN, read at creation, replaces the
+// count from which the density pass takes the warp-cooperative scan, and
+// SPH_GROUP_LANES (1, 8 or 16) sets the lanes of all three kernels.
+void choose_lanes(SphHandle* h, int sms) {
+  const long long n = h->n, per = sms;
+  const int few = n <= 56 * per ? 16 : 8;
+  long long density_max = 384 * per;
+  if (const char* v = std::getenv("SPH_WARP_SCAN_MIN")) density_max = std::atoll(v) - 1;
+  h->lanes_density = n <= density_max ? few : 1;
+  h->lanes_forces = n <= 256 * per ? few : 1;
+  h->lanes_xsph = n <= 128 * per ? few : 1;
+  if (const char* v = std::getenv("SPH_GROUP_LANES")) {
+    const int lanes = std::atoi(v);
+    if (lanes == 1 || lanes == 8 || lanes == 16) h->lanes_xsph = h->lanes_density = h->lanes_forces = lanes;
+  }
+}
 
 // Lets the density kernels take up to 128 KiB of dynamic shared memory (the
 // warp scan's per-warp scratch passes the default 48 KiB at 512 threads) on
@@ -610,6 +631,16 @@ void allow_density_smem() {
   set(reinterpret_cast<const void*>(k_density<ManySim, 0>));
   set(reinterpret_cast<const void*>(k_density<ManySim, 1>));
   set(reinterpret_cast<const void*>(k_density<ManySim, 2>));
+  auto group = [&](auto lanes) {
+    constexpr int G = decltype(lanes)::value;
+    set(reinterpret_cast<const void*>(k_density_group<OneSim, 0, G>));
+    set(reinterpret_cast<const void*>(k_density_group<OneSim, 1, G>));
+    set(reinterpret_cast<const void*>(k_density_group<OneSim, 2, G>));
+    set(reinterpret_cast<const void*>(k_density_group<ManySim, 0, G>));
+    set(reinterpret_cast<const void*>(k_density_group<ManySim, 1, G>));
+    set(reinterpret_cast<const void*>(k_density_group<ManySim, 2, G>));
+  };
+  for (int lanes : {8, 16}) with_lanes(lanes, group);
 }
 
 // Sorting scratch + binning of posU into the cell tables (k_bin or the
@@ -632,27 +663,40 @@ void enqueue_density_only(SphHandle* h) {
   if (h->cl_mode) cudaMemsetAsync(h->cl_count, 0, sizeof(uint32_t), h->st);
   // the warp scan's scratch per warp; closure mode 2 adds a 16-sample network
   // tile per warp (the fused inference)
-  const int warp_scan = h->n >= h->warp_scan_min ? 1 : 0;
-  const size_t smem = warp_scan ? (bs / 32) * sizeof(ScanWarp) : 0;
+  const size_t smem = (bs / 32) * sizeof(ScanWarp);
   const size_t smem_cl = smem + (bs / 32) * kClTileWords * sizeof(uint32_t);
+  if (h->lanes_density > 1) {
+    dispatch(h, false, [&](auto kp) {
+      with_lanes(h->lanes_density, [&](auto lanes) {
+        using KPT = decltype(kp);
+        constexpr int G = decltype(lanes)::value;
+        const int grid = grid_for(h->n, kGroupThreads / G);
+        constexpr size_t smem0 = (kGroupThreads / 32) * sizeof(CoopWarp<G, 2>);
+        constexpr size_t smem1 = (kGroupThreads / 32) * sizeof(CoopWarp<G, 3>);
+        auto launch = [&](auto kernel, size_t smem) {
+          kernel<<<grid, kGroupThreads, smem, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab, h->bc_start,
+                                                       h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount,
+                                                       h->sdf, h->wall_tab, cb, h->slow);
+        };
+        if (h->cl_mode == 2) launch(k_density_group<KPT, 2, G>, smem1 + (kGroupThreads / 32) * kClTileWords * sizeof(uint32_t));
+        else if (h->cl_mode) launch(k_density_group<KPT, 1, G>, smem1);
+        else launch(k_density_group<KPT, 0, G>, smem0);
+      });
+    });
+    h->launches += 1;
+    return;
+  }
   dispatch(h, false, [&](auto kp) {
     using KPT = decltype(kp);
     const int grid = grid_for(h->n, bs);
-    if (h->cl_mode == 2)
-      k_density<KPT, 2><<<grid, bs, smem_cl, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
-                                                     h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
-                                                     h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
-                                                  warp_scan, h->slow);
-    else if (h->cl_mode)
-      k_density<KPT, 1><<<grid, bs, smem, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
-                                                  h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
-                                                  h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
-                                                  warp_scan, h->slow);
-    else
-      k_density<KPT, 0><<<grid, bs, smem, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
-                                                  h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
-                                                  h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
-                                                  warp_scan, h->slow);
+    auto launch = [&](auto kernel, size_t bytes) {
+      kernel<<<grid, bs, bytes, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab, h->bc_start,
+                                         h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount, h->sdf,
+                                         h->wall_tab, cb, h->slow);
+    };
+    if (h->cl_mode == 2) launch(k_density<KPT, 2>, smem_cl);
+    else if (h->cl_mode) launch(k_density<KPT, 1>, smem);
+    else launch(k_density<KPT, 0>, smem);
   });
   h->launches += 1;
 }
@@ -686,6 +730,24 @@ void enqueue_forces(SphHandle* h, float hdt_scale) {
   using namespace sph;
   cudaMemsetAsync(h->red, 0, 2 * sizeof(float) * h->ninst, h->st);
   int bs = h->bs_forces;
+  if (h->lanes_forces > 1) {
+    dispatch(h, false, [&](auto kp) {
+      with_lanes(h->lanes_forces, [&](auto lanes) {
+        using KPT = decltype(kp);
+        constexpr int G = decltype(lanes)::value;
+        auto launch = [&](auto kernel) {
+          kernel<<<grid_for(h->n, kGroupThreads / G), kGroupThreads, 0, h->st>>>(
+              kp, h->n, h->dt, hdt_scale, h->pos, h->vel, h->rf, h->pr, h->id, h->ctab, h->bc_start, h->bc_list,
+              h->bpos, h->bpress, h->acc, h->velout, h->red, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab,
+              h->corr, h->slow);
+        };
+        if (h->cl_mode) launch(k_forces_group<KPT, 1, G>);
+        else launch(k_forces_group<KPT, 0, G>);
+      });
+    });
+    h->launches += 1;
+    return;
+  }
   dispatch(h, false, [&](auto kp) {
     using KPT = decltype(kp);
     auto launch = [&](auto kernel) {
@@ -706,7 +768,15 @@ void enqueue_xsph(SphHandle* h, bool use_list) {
   dispatch(h, false, [&](auto kp) {
     k_xsph_prep<<<grid_for(h->n, 256), 256, 0, h->st>>>(kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec,
                                                          h->err, h->slow);
-    k_xsph_drift<<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec, h->id,
+    if (h->lanes_xsph > 1 && use_list)
+      with_lanes(h->lanes_xsph, [&](auto lanes) {
+        constexpr int G = decltype(lanes)::value;
+        k_xsph_group<decltype(kp), G><<<grid_for(h->n, kGroupThreads / G), kGroupThreads, 0, h->st>>>(
+            kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec, h->id, h->ctab, h->rank_of_lin, h->posU, h->velU,
+            h->idU, h->keyU, h->hist, h->err, h->nbr, h->ncount, h->slow);
+      });
+    else
+      k_xsph_drift<<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec, h->id,
                                                          h->ctab, h->rank_of_lin, h->posU, h->velU, h->idU,
                                                          h->keyU, h->hist, h->err, use_list ? h->nbr : nullptr,
                                                          h->ncount, h->slow);
@@ -955,8 +1025,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     allow_density_smem();
     int sms = 148;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess) sms = 148;
-    h->warp_scan_min = sms * SPH_WARP_SCAN_MIN_PER_SM;
-    if (const char* v = std::getenv("SPH_WARP_SCAN_MIN")) h->warp_scan_min = std::atoi(v);
+    choose_lanes(h, sms);
 #define ALLOC(ptr, cnt) \
   if (ae == cudaSuccess) ae = dalloc(h, &h->ptr, (cnt))
     ALLOC(pos, n); ALLOC(vel, n); ALLOC(velout, n); ALLOC(acc, n);
