@@ -77,8 +77,9 @@ struct SphHandle {
   uint32_t* id = nullptr;
   // unsorted (post-drift) state and sort scratch
   float4 *posU = nullptr, *velU = nullptr;
-  uint32_t *idU = nullptr, *keyU = nullptr, *tmp = nullptr, *tmpid = nullptr;
-  uint32_t *hist = nullptr, *cstart = nullptr, *ccount = nullptr, *cursor = nullptr, *bsum = nullptr;
+  uint32_t *idU = nullptr, *keyU = nullptr, *tmpid = nullptr;
+  uint2 *tmp = nullptr, *crange = nullptr;  // bucket members (particle, cell rank); (start, count) per cell rank
+  uint32_t *hist = nullptr, *bsum = nullptr;
   uint32_t *rank_of_lin = nullptr, *lin_of_rank = nullptr;
   uint2* ctab = nullptr;
   int nbsum = 0;
@@ -597,6 +598,13 @@ void with_lanes(int lanes, F&& f) {
   else f(std::integral_constant<int, 16>());
 }
 
+// A kernel of the step on the handle's stream.
+template <class... P, class... A>
+void launch(SphHandle* h, void (*kernel)(P...), int grid, int block, size_t smem, A... args) {
+  kernel<<<grid, block, smem, h->st>>>(args...);
+  h->launches += 1;
+}
+
 sph::Planes planes(SphHandle* h) { return sph::Planes{h->xyz, h->xyz_stride}; }
 
 // Lanes per particle by size, measured on B200 (the table in sph_group.cuh).
@@ -647,13 +655,16 @@ void allow_density_smem() {
 // xsph kernel fill `hist` first).
 void enqueue_scan_fill(SphHandle* h) {
   using namespace sph;
-  int nbk = h->nbsum;
-  k_scan_reduce<<<nbk, kScanThreads, 0, h->st>>>(h->hist, h->C, h->bsum);
-  k_scan_bsum<<<1, kScanThreads, 0, h->st>>>(h->bsum, nbk);
-  k_scan_apply<<<nbk, kScanThreads, 0, h->st>>>(h->hist, h->C, h->bsum, h->lin_of_rank, h->cstart,
-                                                h->ccount, h->cursor, h->ctab);
-  k_fill<<<grid_for(h->n, 256), 256, 0, h->st>>>(h->n, h->keyU, h->idU, h->cursor, h->tmp, h->tmpid);
-  h->launches += 4;
+  if (h->C <= kScanOne) {
+    launch(h, k_scan_apply<1>, grid_for(h->C, kScanSmallTile), kScanThreads, 0, h->hist, h->C, h->bsum,
+           h->lin_of_rank, h->crange, h->ctab);
+  } else {
+    launch(h, k_scan_reduce, h->nbsum, kScanThreads, 0, h->hist, h->C, h->bsum);
+    if (h->C > kScanTwo) launch(h, k_scan_bsum, 1, kScanThreads, 0, h->bsum, h->nbsum);
+    launch(h, h->C > kScanTwo ? k_scan_apply<3> : k_scan_apply<2>, h->nbsum, kScanThreads, 0, h->hist, h->C, h->bsum,
+           h->lin_of_rank, h->crange, h->ctab);
+  }
+  launch(h, k_fill, grid_for(h->n, 256), 256, 0, h->n, h->keyU, h->idU, h->crange, h->hist, h->tmp, h->tmpid, h->err);
 }
 
 void enqueue_density_only(SphHandle* h) {
@@ -673,32 +684,29 @@ void enqueue_density_only(SphHandle* h) {
         const int grid = grid_for(h->n, kGroupThreads / G);
         constexpr size_t smem0 = (kGroupThreads / 32) * sizeof(CoopWarp<G, 2>);
         constexpr size_t smem1 = (kGroupThreads / 32) * sizeof(CoopWarp<G, 3>);
-        auto launch = [&](auto kernel, size_t smem) {
-          kernel<<<grid, kGroupThreads, smem, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab, h->bc_start,
-                                                       h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount,
-                                                       h->sdf, h->wall_tab, cb, h->slow);
+        auto run = [&](auto kernel, size_t smem) {
+          launch(h, kernel, grid, kGroupThreads, smem, kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
+                 h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
+                 h->slow);
         };
-        if (h->cl_mode == 2) launch(k_density_group<KPT, 2, G>, smem1 + (kGroupThreads / 32) * kClTileWords * sizeof(uint32_t));
-        else if (h->cl_mode) launch(k_density_group<KPT, 1, G>, smem1);
-        else launch(k_density_group<KPT, 0, G>, smem0);
+        if (h->cl_mode == 2) run(k_density_group<KPT, 2, G>, smem1 + (kGroupThreads / 32) * kClTileWords * sizeof(uint32_t));
+        else if (h->cl_mode) run(k_density_group<KPT, 1, G>, smem1);
+        else run(k_density_group<KPT, 0, G>, smem0);
       });
     });
-    h->launches += 1;
     return;
   }
   dispatch(h, false, [&](auto kp) {
     using KPT = decltype(kp);
     const int grid = grid_for(h->n, bs);
-    auto launch = [&](auto kernel, size_t bytes) {
-      kernel<<<grid, bs, bytes, h->st>>>(kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab, h->bc_start,
-                                         h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount, h->sdf,
-                                         h->wall_tab, cb, h->slow);
+    auto run = [&](auto kernel, size_t bytes) {
+      launch(h, kernel, grid, bs, bytes, kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab, h->bc_start,
+             h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab, cb, h->slow);
     };
-    if (h->cl_mode == 2) launch(k_density<KPT, 2>, smem_cl);
-    else if (h->cl_mode) launch(k_density<KPT, 1>, smem);
-    else launch(k_density<KPT, 0>, smem);
+    if (h->cl_mode == 2) run(k_density<KPT, 2>, smem_cl);
+    else if (h->cl_mode) run(k_density<KPT, 1>, smem);
+    else run(k_density<KPT, 0>, smem);
   });
-  h->launches += 1;
 }
 
 // boundary.rs:87-123: the Adami boundary pressure (a boundary particle without
@@ -709,16 +717,14 @@ void enqueue_adami(SphHandle* h) {
   if (h->wlist) {
     const int P = h->n >= 1000000 ? 16 : 8;  // between 250k and 2M particles the two cross (k_wall_scatter)
     dispatch(h, false, [&](auto kp) {
-      k_wall_scatter<<<grid_for(h->n, 8 * P), 256, 0, h->st>>>(kp, h->n, P, h->pos, h->nbr, h->ncount, h->bc_start,
-                                                               h->bc_list, h->bpos, h->wcount, h->wlist, h->err);
+      launch(h, k_wall_scatter<decltype(kp)>, grid_for(h->n, 8 * P), 256, 0, kp, h->n, P, h->pos, h->nbr, h->ncount,
+             h->bc_start, h->bc_list, h->bpos, h->wcount, h->wlist, h->err);
     });
-    h->launches += 1;
   }
   dispatch(h, true, [&](auto kp) {
-    k_adami<<<grid_for(h->nb, kAdamiWarps * 4), kAdamiWarps * 32, 0, h->st>>>(
-        kp, h->nb, h->bpos, h->bpress, h->pos, h->rf, h->pr, h->id, h->ctab, h->err, h->wcount, h->wlist);
+    launch(h, k_adami<decltype(kp)>, grid_for(h->nb, kAdamiWarps * 4), kAdamiWarps * 32, 0, kp, h->nb, h->bpos,
+           h->bpress, h->pos, h->rf, h->pr, h->id, h->ctab, h->err, h->wcount, h->wlist);
   });
-  h->launches += 1;
 }
 
 void enqueue_density_adami(SphHandle* h) {
@@ -726,77 +732,76 @@ void enqueue_density_adami(SphHandle* h) {
   enqueue_adami(h);
 }
 
+// `red` is clear when it runs (clear_red, or k_reorder).
 void enqueue_forces(SphHandle* h, float hdt_scale) {
   using namespace sph;
-  cudaMemsetAsync(h->red, 0, 2 * sizeof(float) * h->ninst, h->st);
-  int bs = h->bs_forces;
-  if (h->lanes_forces > 1) {
-    dispatch(h, false, [&](auto kp) {
-      with_lanes(h->lanes_forces, [&](auto lanes) {
-        using KPT = decltype(kp);
-        constexpr int G = decltype(lanes)::value;
-        auto launch = [&](auto kernel) {
-          kernel<<<grid_for(h->n, kGroupThreads / G), kGroupThreads, 0, h->st>>>(
-              kp, h->n, h->dt, hdt_scale, h->pos, h->vel, h->rf, h->pr, h->id, h->ctab, h->bc_start, h->bc_list,
-              h->bpos, h->bpress, h->acc, h->velout, h->red, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab,
-              h->corr, h->slow);
-        };
-        if (h->cl_mode) launch(k_forces_group<KPT, 1, G>);
-        else launch(k_forces_group<KPT, 0, G>);
-      });
-    });
-    h->launches += 1;
-    return;
-  }
   dispatch(h, false, [&](auto kp) {
     using KPT = decltype(kp);
-    auto launch = [&](auto kernel) {
-      kernel<<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, hdt_scale, h->pos, h->vel, h->rf, h->pr, h->id,
-                                                  h->ctab, h->bc_start, h->bc_list, h->bpos, h->bpress, h->acc,
-                                                  h->velout, h->red, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab,
-                                                  h->corr, h->slow);
+    auto run = [&](auto kernel, int grid, int block) {
+      launch(h, kernel, grid, block, 0, kp, h->n, h->dt, hdt_scale, h->pos, h->vel, h->rf, h->pr, h->id, h->ctab,
+             h->bc_start, h->bc_list, h->bpos, h->bpress, h->acc, h->velout, h->red, h->err, h->nbr, h->ncount,
+             h->sdf, h->wall_tab, h->corr, h->slow);
     };
-    if (h->cl_mode) launch(k_forces<KPT, 1>);
-    else launch(k_forces<KPT, 0>);
+    if (h->lanes_forces > 1) {
+      with_lanes(h->lanes_forces, [&](auto lanes) {
+        constexpr int G = decltype(lanes)::value;
+        const int grid = grid_for(h->n, kGroupThreads / G);
+        if (h->cl_mode) run(k_forces_group<KPT, 1, G>, grid, kGroupThreads);
+        else run(k_forces_group<KPT, 0, G>, grid, kGroupThreads);
+      });
+    } else {
+      const int bs = h->bs_forces;
+      if (h->cl_mode) run(k_forces<KPT, 1>, grid_for(h->n, bs), bs);
+      else run(k_forces<KPT, 0>, grid_for(h->n, bs), bs);
+    }
   });
-  h->launches += 1;
 }
 
-void enqueue_xsph(SphHandle* h, bool use_list) {
+void clear_red(SphHandle* h) { cudaMemsetAsync(h->red, 0, 2 * sizeof(float) * h->ninst, h->st); }
+
+void enqueue_dt_finalize(SphHandle* h, float* out) {
+  launch(h, sph::k_dt_finalize, grid_for(h->ninst, 128), 128, 0, h->ninst, h->hcc, h->red, out);
+}
+
+// Kick 1, XSPH, drift and binning. With `auto_dt` the step's dt comes from the
+// last step's maxima (in h->red), else it is in h->dt.
+void enqueue_xsph(SphHandle* h, bool use_list, bool auto_dt = false) {
   using namespace sph;
-  int bs = h->bs_xsph;
-  dispatch(h, false, [&](auto kp) {
-    k_xsph_prep<<<grid_for(h->n, 256), 256, 0, h->st>>>(kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec,
-                                                         h->err, h->slow);
-    if (h->lanes_xsph > 1 && use_list)
+  if (h->lanes_xsph > 1 && use_list) {
+    dispatch(h, false, [&](auto kp) {
       with_lanes(h->lanes_xsph, [&](auto lanes) {
         constexpr int G = decltype(lanes)::value;
-        k_xsph_group<decltype(kp), G><<<grid_for(h->n, kGroupThreads / G), kGroupThreads, 0, h->st>>>(
-            kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec, h->id, h->ctab, h->rank_of_lin, h->posU, h->velU,
-            h->idU, h->keyU, h->hist, h->err, h->nbr, h->ncount, h->slow);
+        launch(h, k_xsph_group<decltype(kp), G>, grid_for(h->n, kGroupThreads / G), kGroupThreads, 0, kp, h->n, h->dt,
+               auto_dt ? h->red : nullptr, h->pos, h->velout, h->acc, h->id, h->ctab, h->rank_of_lin, h->posU,
+               h->velU, h->idU, h->keyU, h->hist, h->err, h->nbr, h->ncount);
       });
-    else
-      k_xsph_drift<<<grid_for(h->n, bs), bs, 0, h->st>>>(kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec, h->id,
-                                                         h->ctab, h->rank_of_lin, h->posU, h->velU, h->idU,
-                                                         h->keyU, h->hist, h->err, use_list ? h->nbr : nullptr,
-                                                         h->ncount, h->slow);
+    });
+    return;
+  }
+  if (auto_dt) enqueue_dt_finalize(h, h->dt);
+  const int bs = h->bs_xsph;
+  dispatch(h, false, [&](auto kp) {
+    using KPT = decltype(kp);
+    launch(h, k_xsph_prep<KPT>, grid_for(h->n, 256), 256, 0, kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec,
+           h->err, h->slow);
+    launch(h, k_xsph_drift<KPT>, grid_for(h->n, bs), bs, 0, kp, h->n, h->dt, h->pos, h->velout, h->acc, h->xrec,
+           h->id, h->ctab, h->rank_of_lin, h->posU, h->velU, h->idU, h->keyU, h->hist, h->err,
+           use_list ? h->nbr : nullptr, h->ncount, h->slow);
   });
-  h->launches += 2;
 }
 
+// The sort; it also clears `red` for enqueue_forces.
 void enqueue_sort(SphHandle* h) {
   using namespace sph;
   enqueue_scan_fill(h);
-  k_reorder<<<grid_for(h->n, 256), 256, 0, h->st>>>(h->n, h->tmp, h->tmpid, h->keyU, h->cstart, h->ccount,
-                                                    h->posU, h->velU, h->pos, h->vel, h->rv, h->id, h->err,
-                                                    nullptr, nullptr, nullptr, nullptr, nullptr, planes(h));
-  h->launches += 1;
+  launch(h, k_reorder, grid_for(h->n, 256), 256, 0, h->n, h->tmp, h->tmpid, h->crange, h->posU, h->velU, h->pos,
+         h->vel, h->rv, h->id, h->err, nullptr, nullptr, nullptr, nullptr, nullptr, planes(h), h->red, 2 * h->ninst);
 }
 
 // lib.rs:287-335 after the bootstrap: kick1+XSPH+drift+clamp, grid + reorder,
 // density, boundary pressure, forces + kick2.
-void enqueue_body(SphHandle* h, bool use_list) {
-  enqueue_xsph(h, use_list);
+void enqueue_body(SphHandle* h, bool use_list, bool auto_dt = false) {
+  enqueue_xsph(h, use_list, auto_dt);
   enqueue_sort(h);
   enqueue_density_adami(h);
   enqueue_forces(h, 1.0f);
@@ -805,12 +810,8 @@ void enqueue_body(SphHandle* h, bool use_list) {
 // lib.rs:295-298: compute_forces(dt) once before the first step.
 void enqueue_bootstrap(SphHandle* h) {
   enqueue_density_adami(h);
+  clear_red(h);
   enqueue_forces(h, 0.0f);
-}
-
-void enqueue_dt_finalize(SphHandle* h, float* out) {
-  sph::k_dt_finalize<<<grid_for(h->ninst, 128), 128, 0, h->st>>>(h->ninst, h->hcc, h->red, out);
-  h->launches += 1;
 }
 
 void enqueue_set_dt(SphHandle* h, float dt) {
@@ -822,8 +823,7 @@ int capture(SphHandle* h, bool with_finalize, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   uint64_t before = h->launches;
   SPH_TRY(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
-  if (with_finalize) enqueue_dt_finalize(h, h->dt);
-  enqueue_body(h, true);
+  enqueue_body(h, true, with_finalize);
   cudaError_t e = cudaStreamEndCapture(h->st, &g);
   if (e != cudaSuccess) return cuda_status(h, e, "cudaStreamEndCapture");
   h->body_kernels = (int)(h->launches - before);
@@ -1031,7 +1031,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     ALLOC(pos, n); ALLOC(vel, n); ALLOC(velout, n); ALLOC(acc, n);
     ALLOC(rv, n); ALLOC(rf, n); ALLOC(pr, n); ALLOC(id, n);
     ALLOC(posU, n); ALLOC(velU, n); ALLOC(idU, n); ALLOC(keyU, n); ALLOC(tmp, n); ALLOC(tmpid, n);
-    ALLOC(hist, C); ALLOC(cstart, C); ALLOC(ccount, C); ALLOC(cursor, C); ALLOC(bsum, h->nbsum);
+    ALLOC(hist, C); ALLOC(crange, C); ALLOC(bsum, h->nbsum);
     ALLOC(rank_of_lin, C); ALLOC(lin_of_rank, C); ALLOC(ctab, C);
     ALLOC(bpos, nb); ALLOC(bpress, nb); ALLOC(wcount, nb); ALLOC(bc_start, C + 1);
     ALLOC(dt, ninst); ALLOC(dt_query, ninst); ALLOC(red, 2 * ninst); ALLOC(err, 1); ALLOC(hcc, ninst);
@@ -1299,11 +1299,8 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     });
     h->launches += 1;
     enqueue_scan_fill(h);
-    k_reorder<<<grid_for(h->n, 256), 256, 0, h->st>>>(h->n, h->tmp, h->tmpid, h->keyU, h->cstart,
-                                                      h->ccount, h->posU, h->velU, h->pos, h->vel, h->rv,
-                                                      h->id, h->err, accU, h->acc, prU, h->pr, h->velout,
-                                                      planes(h));
-    h->launches += 1;
+    launch(h, k_reorder, grid_for(h->n, 256), 256, 0, h->n, h->tmp, h->tmpid, h->crange, h->posU, h->velU, h->pos,
+           h->vel, h->rv, h->id, h->err, accU, h->acc, prU, h->pr, h->velout, planes(h), nullptr, 0);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);

@@ -112,15 +112,19 @@ __device__ __forceinline__ void group_candidates(const Group<G>& g, uint32_t q0,
 // ---------------------------------------------------------------------------
 // XSPH + drift (k_xsph_drift's work)
 // ---------------------------------------------------------------------------
+// The neighbours' half-kicked velocities (k_xsph_prep's records in the thread
+// form) are computed here from velocity and acceleration: a launch less, where
+// launches count. With `red` the kernel also computes the step's dt from the
+// last step's maxima, for every instance's own particles, and stores it.
 template <class KP, int G>
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
-k_xsph_group(KP kp, int n, const float* __restrict__ dtp, const float4* __restrict__ pos,
-             const float4* __restrict__ velout, const float4* __restrict__ acc, const float4* __restrict__ rec,
+k_xsph_group(KP kp, int n, float* __restrict__ dtp, const float* __restrict__ red, const float4* __restrict__ pos,
+             const float4* __restrict__ velout, const float4* __restrict__ acc,
              const uint32_t* __restrict__ id, const uint2* __restrict__ ctab,
              const uint32_t* __restrict__ rank_of_lin, float4* __restrict__ posU, float4* __restrict__ velU,
              uint32_t* __restrict__ idU, uint32_t* __restrict__ keyU, uint32_t* __restrict__ hist,
              const uint32_t* __restrict__ err, const uint32_t* __restrict__ nbr,
-             const uint32_t* __restrict__ ncount, const uint32_t* __restrict__ slow) {
+             const uint32_t* __restrict__ ncount) {
   constexpr int U = kRounds, CH = kChunkOf<G>;
   __shared__ GroupTerms<3, CH> s_terms[kGroupThreads / G];
   const Group<G> g;
@@ -129,49 +133,65 @@ k_xsph_group(KP kp, int n, const float* __restrict__ dtp, const float4* __restri
   const bool live = slot < n && !*err;
   const int i = live ? slot : 0;
   const SimConst& k = kp.at(i);
-  const float dt = dtp[k.inst];
+  float dt;
+  if (red) {
+    dt = cfl_dt(k.h, k.c, k.cfl, red[2 * k.inst], red[2 * k.inst + 1]);
+    if (live && g.sub == 0 && kp.first(i)) dtp[k.inst] = dt;
+  } else {
+    dt = dtp[k.inst];
+  }
   const float4 pi = pos[i];
   const float4 vi = velout[i];
   const float4 ai = acc[i];
   const float hdt = 0.5f * dt;
-  float vx = vi.x + ai.x * hdt;
-  float vy = vi.y + ai.y * hdt;
-  float vz = vi.z + ai.z * hdt;
+  const float vx = vi.x + ai.x * hdt;
+  const float vy = vi.y + ai.y * hdt;
+  const float vz = vi.z + ai.z * hdt;
   float sum = 0.0f;  // lanes 0..2: the components of the XSPH sum
   const bool xsph = live && (k.flags & kFlagXsph);
-  const uint32_t counts = xsph ? (!slow[k.inst] ? __ldg(&ncount[i]) : kRescanBit) : 0u;
+  const uint32_t counts = xsph ? (k.fast ? __ldg(&ncount[i]) : kRescanBit) : 0u;
   const bool listed = counts_listed(counts);
   const uint32_t mine = listed ? counts_neighbours(counts) : 0u;
   const uint32_t most = __reduce_max_sync(0xffffffffu, mine);
+  // the quotient's operands are watched here: the largest density, and whether
+  // a mass lies outside the range
+  float rho_max = vi.w;
+  bool odd = false;
   GroupList<G> list(nbr, n, i, g.sub);
   for (uint32_t c0 = 0; c0 < most; c0 += CH) {
     // the entries past the list's end are in bounds and not used: their lanes
     // gather the particle itself and put zeros
-    float4 pj[U], vh[U];
+    float4 pj[U], vj[U], aj[U];
     uint32_t s[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) s[u] = list.next();
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (!(c0 + u * G + g.sub < mine)) s[u] = (uint32_t)i;
-      ld_record(rec + 2 * (size_t)s[u], pj[u], vh[u]);
+      pj[u] = __ldg(&pos[s[u]]);
+      vj[u] = __ldg(&velout[s[u]]);
+      aj[u] = __ldg(&acc[s[u]]);
     }
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const float dx = pi.x - pj[u].x, dy = pi.y - pj[u].y, dz = pi.z - pj[u].z;
-      const float factor = xsph_factor(dx * dx + dy * dy + dz * dz, pj[u].w, vi.w + vh[u].w, k);
+      const float factor = xsph_factor(dx * dx + dy * dy + dz * dz, 2.0f * pj[u].w, vi.w + vj[u].w, k);
+      const float m = fabsf(pj[u].w);
+      rho_max = fmaxf(rho_max, vj[u].w);
+      odd = odd || !(m == 0.0f || (m >= kMassMin && m <= kMassMax));
       const bool in = c0 + u * G + g.sub < mine;
-      T.t[0][u * G + g.sub] = in ? factor * (vh[u].x - vx) : 0.0f;
-      T.t[1][u * G + g.sub] = in ? factor * (vh[u].y - vy) : 0.0f;
-      T.t[2][u * G + g.sub] = in ? factor * (vh[u].z - vz) : 0.0f;
+      T.t[0][u * G + g.sub] = in ? factor * ((vj[u].x + aj[u].x * hdt) - vx) : 0.0f;
+      T.t[1][u * G + g.sub] = in ? factor * ((vj[u].y + aj[u].y * hdt) - vy) : 0.0f;
+      T.t[2][u * G + g.sub] = in ? factor * ((vj[u].z + aj[u].z * hdt) - vz) : 0.0f;
     }
     __syncwarp();
     if (g.sub < 3 && c0 < mine) sum = add_terms(T, g.sub, min(mine - c0, (uint32_t)CH), sum);
     __syncwarp();
   }
+  odd = g.bits(__ballot_sync(0xffffffffu, odd || rho_max > kRhoMax)) != 0u;
   float sx = g.get(sum, 0), sy = g.get(sum, 1), sz = g.get(sum, 2);
-  if (xsph && (!listed || !finite3(sx, sy, sz))) {
-    const Sum3 e = xsph_exact(kp.ref(i), i, pi, make_float4(vx, vy, vz, vi.w), pos, rec, ctab);
+  if (xsph && (!listed || odd || !finite3(sx, sy, sz))) {
+    const Sum3 e = xsph_exact(kp.ref(i), i, pi, make_float4(vx, vy, vz, vi.w), hdt, pos, velout, acc, ctab);
     sx = e.x;
     sy = e.y;
     sz = e.z;
