@@ -4,6 +4,7 @@
 // buffers and CUDA graphs. The step body (9 kernels) is captured once into a
 // graph and replayed; dt lives in device memory so the graph never changes.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdlib>
@@ -124,22 +125,28 @@ struct SphHandle {
   float *cl_feat = nullptr, *cl_rho = nullptr, *cl_wf = nullptr;
   float4* corr = nullptr;
   __nv_bfloat16* cl_wb = nullptr;
-  // scalars
-  float *dt = nullptr, *dt_query = nullptr, *red = nullptr;
+  // scalars, one allocation so that one copy reads a result with the error
+  // flags: (mass, energy) sums, density variation, flags, the step's dt and
+  // the queried one per instance
+  double* me = nullptr;
+  float* var = nullptr;
   uint32_t* err = nullptr;
+  float *dt = nullptr, *dt_query = nullptr, *red = nullptr;
   uint32_t* slow = nullptr;  // per instance: its pair sums take the general operations (k_xsph_prep, k_density)
   // metrics
   int nparts = 0;
-  double *part_m = nullptr, *part_e = nullptr, *me = nullptr;
-  float *part_var = nullptr, *var = nullptr;
+  double *part_m = nullptr, *part_e = nullptr;
+  float* part_var = nullptr;
+  uint32_t* metrics_done = nullptr;
   unsigned long long* bad = nullptr;
   // checkpoint
   float4 *ck_pos = nullptr, *ck_velout = nullptr, *ck_acc = nullptr;
   float* ck_pr = nullptr;
   uint32_t* ck_slot = nullptr;
-  // readback staging
+  // readback staging: 12 planes in original order, then the fluid types
   float* stage = nullptr;
   uint8_t* stage_ft = nullptr;
+  bool counted = false;  // among the device's live handles (HostStage)
   // diagnostics scratch
   uint32_t* diag = nullptr;
   // geometry for force extraction
@@ -842,15 +849,156 @@ void drop_graphs(SphHandle* h) {
   h->g_opt = nullptr;
 }
 
-int check_device_flags(SphHandle* h) {
-  uint32_t e = 0;
-  SPH_TRY(h, cudaMemcpyAsync(&e, h->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->st));
-  SPH_TRY(h, cudaStreamSynchronize(h->st));
+int flags_status(SphHandle* h, uint32_t e) {
   if (e & sph::kErrCellCap)
     return set_err(h, SPH_ERR_CAPACITY, "a grid cell exceeded 4096 particles");
   if (e & sph::kErrAdamiCap)
     return set_err(h, SPH_ERR_CAPACITY, "a boundary particle has more than 256 fluid particles in support");
   return SPH_OK;
+}
+
+int check_device_flags(SphHandle* h) {
+  uint32_t e = 0;
+  SPH_TRY(h, cudaMemcpyAsync(&e, h->err, sizeof(uint32_t), cudaMemcpyDeviceToHost, h->st));
+  SPH_TRY(h, cudaStreamSynchronize(h->st));
+  return flags_status(h, e);
+}
+
+// The step's dt (query: the queried one) of every instance and the error
+// flags, in one copy. Waits for the stream.
+int read_dt(SphHandle* h, bool query, int count, float* dt_out) {
+  const size_t n = (size_t)h->ninst;
+  const size_t words = 1 + (query ? 2 * n : (size_t)count);
+  std::unique_ptr<float[]> many;
+  float few[65];
+  float* w = few;
+  if (words > 65) {
+    many.reset(new (std::nothrow) float[words]);
+    if (!many) return set_err(h, SPH_ERR_OOM, "host memory");
+    w = many.get();
+  }
+  SPH_TRY(h, cudaMemcpyAsync(w, h->err, words * sizeof(float), cudaMemcpyDeviceToHost, h->st));
+  SPH_TRY(h, cudaStreamSynchronize(h->st));
+  uint32_t e;
+  std::memcpy(&e, w, sizeof e);
+  std::memcpy(dt_out, w + 1 + (query ? n : 0), (size_t)count * sizeof(float));
+  return flags_status(h, e);
+}
+
+// Page-locked memory that reads of a device's particle state pass through, one
+// per device, of at most kStageBytes. A copy per array into pageable memory
+// costs a driver call each and a driver thread's copy of every page; here the
+// staging area comes over in pieces, and the next piece is on its way while the
+// host moves the last to its arrays. The first touch of a caller's fresh pages
+// bounds it, hence several host threads for a large read; below 8 MB their
+// start costs more than they give. One read through the Python mirror (whose
+// arrays are backed with huge pages), before and now: 2k particles 228 -> 74
+// us, 31k 530 -> 195, 250k 2150 -> 830, 600k 4900 -> 1400, 2M 14,500 -> 3950.
+// A reader that finds the staging taken by another thread copies directly. It
+// is given back when the device's last handle is destroyed.
+constexpr size_t kStagePiece = 1 << 20, kStageOneThread = 8 << 20;
+constexpr unsigned kStageThreads = 4;
+constexpr size_t kStageBytes = kStageThreads * 2 * kStagePiece;
+struct HostStage {
+  std::mutex mu;
+  char* p = nullptr;
+  size_t bytes = 0;
+  cudaStream_t st[kStageThreads] = {};
+  int handles = 0;
+  void give_back() {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    bytes = 0;
+    for (cudaStream_t& s : st) {
+      if (s) cudaStreamDestroy(s);
+      s = nullptr;
+    }
+  }
+  bool room(size_t want) {  // page-locked memory for a read of `want` bytes
+    want = std::min(kStageBytes, (want + 65535) / 65536 * 65536);
+    if (bytes >= want) return true;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    bytes = 0;
+    if (cudaHostAlloc((void**)&p, want, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      p = nullptr;
+      return false;
+    }
+    bytes = want;
+    return true;
+  }
+};
+HostStage* host_stage(int dev) {
+  static HostStage stages[64];
+  return dev >= 0 && dev < 64 ? &stages[dev] : nullptr;
+}
+void count_handle(SphHandle* h, int by) {
+  HostStage* s = host_stage(h->dev);
+  if (!s || h->counted == (by > 0)) return;
+  h->counted = by > 0;
+  std::lock_guard<std::mutex> lock(s->mu);
+  s->handles += by;
+  if (s->handles == 0) s->give_back();
+}
+
+struct ReadPart {
+  void* dst;
+  size_t off, bytes;  // its range of the device staging area
+};
+
+// Copies the device staging area (`span` bytes at src, ready) to the pageable
+// arrays of `parts`, and `host_bytes` of host memory beside it. False: not
+// done, the caller copies directly.
+bool read_through_stage(SphHandle* h, const char* src, size_t span, const ReadPart* parts, size_t nparts,
+                        void* host_dst, const void* host_src, size_t host_bytes, cudaError_t* err) {
+  HostStage* s = host_stage(h->dev);
+  if (!s) return false;
+  std::unique_lock<std::mutex> lock(s->mu, std::try_to_lock);
+  if (!lock.owns_lock()) return false;
+  const size_t pieces = (span + kStagePiece - 1) / kStagePiece;
+  const unsigned T = span <= kStageOneThread ? 1u : std::min(kStageThreads, std::max(1u, std::thread::hardware_concurrency()));
+  if (!s->room(pieces <= 1 ? span : T * 2 * kStagePiece)) return false;
+  for (unsigned t = 0; t < T; ++t)
+    if (!s->st[t] && cudaStreamCreateWithFlags(&s->st[t], cudaStreamNonBlocking) != cudaSuccess) {
+      cudaGetLastError();
+      s->st[t] = nullptr;
+      return false;
+    }
+  std::atomic<size_t> next{0};
+  std::atomic<int> bad{(int)cudaSuccess};
+  run_threads(T, [&](unsigned t) {
+    if (cudaSetDevice(h->dev) != cudaSuccess) {
+      bad = (int)cudaErrorInvalidDevice;
+      return;
+    }
+    char* slot[2] = {s->p + 2 * t * kStagePiece, s->p + (2 * t + 1) * kStagePiece};
+    size_t ahead = pieces;  // the piece on its way into slot[w]; none at first
+    int w = 1;  // the first piece goes to slot 0
+    for (;;) {
+      size_t q = next.fetch_add(1);
+      if (q >= pieces || bad.load() != (int)cudaSuccess) q = pieces;
+      cudaError_t e = ahead < pieces ? cudaStreamSynchronize(s->st[t]) : cudaSuccess;
+      if (e == cudaSuccess && q < pieces)
+        e = cudaMemcpyAsync(slot[w ^ 1], src + q * kStagePiece, std::min(kStagePiece, span - q * kStagePiece),
+                            cudaMemcpyDeviceToHost, s->st[t]);
+      if (e != cudaSuccess) bad = (int)e;
+      if (ahead < pieces && e == cudaSuccess) {
+        const size_t lo = ahead * kStagePiece, hi = std::min(span, lo + kStagePiece);
+        for (size_t k = 0; k < nparts; ++k) {
+          const size_t a = std::max(lo, parts[k].off), b = std::min(hi, parts[k].off + parts[k].bytes);
+          if (a < b) std::memcpy((char*)parts[k].dst + (a - parts[k].off), slot[w] + (a - lo), b - a);
+        }
+      }
+      if (q == pieces || e != cudaSuccess) break;
+      ahead = q;
+      w ^= 1;
+    }
+    if (t == 0 && host_bytes) std::memcpy(host_dst, host_src, host_bytes);
+  });
+  for (unsigned t = 0; t < T && bad.load() != (int)cudaSuccess; ++t) cudaStreamSynchronize(s->st[t]);
+  *err = (cudaError_t)bad.load();
+  return true;
 }
 
 void ensure_red(SphHandle* h) {
@@ -1034,10 +1182,15 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     ALLOC(hist, C); ALLOC(crange, C); ALLOC(bsum, h->nbsum);
     ALLOC(rank_of_lin, C); ALLOC(lin_of_rank, C); ALLOC(ctab, C);
     ALLOC(bpos, nb); ALLOC(bpress, nb); ALLOC(wcount, nb); ALLOC(bc_start, C + 1);
-    ALLOC(dt, ninst); ALLOC(dt_query, ninst); ALLOC(red, 2 * ninst); ALLOC(err, 1); ALLOC(hcc, ninst);
-    ALLOC(part_m, h->nparts); ALLOC(part_e, h->nparts); ALLOC(part_var, h->nparts); ALLOC(me, 2);
-    ALLOC(var, 1); ALLOC(bad, 1);
-    ALLOC(stage, 12 * n); ALLOC(stage_ft, n); ALLOC(diag, 2);
+    ALLOC(me, 3 + ninst); ALLOC(red, 2 * ninst); ALLOC(hcc, ninst);
+    ALLOC(part_m, h->nparts); ALLOC(part_e, h->nparts); ALLOC(part_var, h->nparts);
+    ALLOC(bad, 1); ALLOC(metrics_done, 1);
+    ALLOC(stage, 12 * n + (n + 3) / 4); ALLOC(diag, 2);
+    h->stage_ft = reinterpret_cast<uint8_t*>(h->stage + 12 * n);
+    h->var = reinterpret_cast<float*>(h->me + 2);
+    h->err = reinterpret_cast<uint32_t*>(h->var + 1);
+    h->dt = h->var + 2;
+    h->dt_query = h->dt + ninst;
     ALLOC(nbr, (size_t)sph::kNbrCap * n); ALLOC(ncount, n); ALLOC(xrec, 2 * n);
     h->xyz_stride = ((size_t)n + 3) / 4 * 4 + 4;  // aligned groups of 4 may read past the last slot
     ALLOC(xyz, 3 * h->xyz_stride);
@@ -1286,6 +1439,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   if (e == cudaSuccess) e = cudaMemsetAsync(h->hist, 0, C * sizeof(uint32_t), h->st);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->bpress, 0, std::max<size_t>(1, nb) * sizeof(float), h->st);
   if (e == cudaSuccess) e = cudaMemsetAsync(h->err, 0, sizeof(uint32_t), h->st);
+  if (e == cudaSuccess) e = cudaMemsetAsync(h->metrics_done, 0, sizeof(uint32_t), h->st);
   std::vector<uint32_t> slow(ninst);
   for (int q = 0; q < ninst; ++q) slow[q] = h->ktab_h[q].fast ? 0u : 1u;
   up(h->slow, slow.data(), ninst * sizeof(uint32_t));
@@ -1315,6 +1469,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   int st = check_device_flags(h);
   if (st != SPH_OK) return fail(st);
   trace.mark("done");
+  count_handle(h, 1);
   *out = h;
   return SPH_OK;
 }
@@ -1372,6 +1527,7 @@ void sph_destroy(SphHandle* h) {
   cudaSetDevice(h->dev);
   if (h->st) cudaStreamSynchronize(h->st);
   free_all(h);
+  count_handle(h, -1);
   delete h;
 }
 
@@ -1444,11 +1600,7 @@ int sph_step_auto(SphHandle* h, int nsteps, float* dt_out) {
     h->list_valid = true;
     h->red_valid = true;
   }
-  if (dt_out) {
-    SPH_TRY(h, cudaMemcpyAsync(dt_out, h->dt, sizeof(float), cudaMemcpyDeviceToHost, h->st));
-    SPH_TRY(h, cudaStreamSynchronize(h->st));
-    return check_device_flags(h);
-  }
+  if (dt_out) return read_dt(h, false, 1, dt_out);
   return cuda_status(h, cudaGetLastError(), "sph_step_auto");
 }
 
@@ -1462,9 +1614,7 @@ int sph_compute_timestep(SphHandle* h, float* dt_out) {
   }
   ensure_red(h);
   enqueue_dt_finalize(h, h->dt_query);
-  SPH_TRY(h, cudaMemcpyAsync(dt_out, h->dt_query, sizeof(float), cudaMemcpyDeviceToHost, h->st));
-  SPH_TRY(h, cudaStreamSynchronize(h->st));
-  return check_device_flags(h);
+  return read_dt(h, true, 1, dt_out);
 }
 
 int sph_step_profiled(SphHandle* h, float dt, SphStepProfile* prof) {
@@ -1520,13 +1670,37 @@ int sph_read_particles(SphHandle* h, SphParticlesMut* o) {
   sph::k_unsort<<<grid_for(h->n, 256), 256, 0, h->st>>>(h->n, h->pos, h->velout, h->acc, h->pr, h->id,
                                                        h->stage, h->stage_ft);
   h->launches += 1;
+  SPH_TRY(h, cudaGetLastError());
+  uint32_t flags = 0;  // after the work on the stream: the staging's own streams may read
+  SPH_TRY(h, cudaMemcpyAsync(&flags, h->err, sizeof flags, cudaMemcpyDeviceToHost, h->st));
+  SPH_TRY(h, cudaStreamSynchronize(h->st));
+  bool pageable = true;  // page-locked or device arrays take direct copies
+  for (int f = 0; f < 13 && pageable; ++f) {
+    const void* p = f < 12 ? (const void*)dst[f] : (const void*)o->fluid_type;
+    cudaPointerAttributes a;
+    if (p && cudaPointerGetAttributes(&a, p) == cudaSuccess) pageable = a.type == cudaMemoryTypeUnregistered;
+  }
+  cudaGetLastError();
+  cudaError_t e = cudaSuccess;
+  bool done = false;
+  if (pageable) {
+    ReadPart parts[13];
+    for (int f = 0; f < 12; ++f) parts[f] = {dst[f], f * n * sizeof(float), n * sizeof(float)};
+    parts[12] = {o->fluid_type, 12 * n * sizeof(float), n};
+    done = read_through_stage(h, (const char*)h->stage, n * (12 * sizeof(float) + 1), parts, o->fluid_type ? 13 : 12,
+                              o->temperature, h->temperature.data(), o->temperature ? n * sizeof(float) : 0, &e);
+  }
+  if (done) {
+    if (e != cudaSuccess) return cuda_status(h, e, "sph_read_particles");
+    return flags_status(h, flags);
+  }
   for (int f = 0; f < 12; ++f)
     SPH_TRY(h, cudaMemcpyAsync(dst[f], h->stage + f * n, n * sizeof(float), cudaMemcpyDeviceToHost, h->st));
   if (o->fluid_type)
     SPH_TRY(h, cudaMemcpyAsync(o->fluid_type, h->stage_ft, n, cudaMemcpyDeviceToHost, h->st));
   SPH_TRY(h, cudaStreamSynchronize(h->st));
   if (o->temperature) std::memcpy(o->temperature, h->temperature.data(), n * sizeof(float));
-  return check_device_flags(h);
+  return flags_status(h, flags);
 }
 
 int sph_read_boundary_pressure(SphHandle* h, float* out, size_t nb) {
@@ -1540,10 +1714,8 @@ int sph_read_boundary_pressure(SphHandle* h, float* out, size_t nb) {
 namespace {
 // FP64 mass / energy sums and the maximum density variation into h->me, h->var
 void enqueue_metrics(SphHandle* h) {
-  sph::k_metrics_partial<<<h->nparts, sph::kMetricThreads, 0, h->st>>>(h->k, h->n, h->pos, h->velout, h->id,
-                                                                     h->part_m, h->part_e, h->part_var);
-  sph::k_metrics_final<<<1, 32, 0, h->st>>>(h->nparts, h->part_m, h->part_e, h->part_var, h->me, h->var);
-  h->launches += 2;
+  launch(h, sph::k_metrics, h->nparts, sph::kMetricThreads, 0, h->k, h->n, h->pos, h->velout, h->id, h->part_m,
+         h->part_e, h->part_var, h->metrics_done, h->me, h->var);
 }
 
 cudaError_t ensure_ck(SphHandle* h) {
@@ -1579,19 +1751,22 @@ void enqueue_restore_ck(SphHandle* h) {
 int sph_error_metrics(SphHandle* h, SphErrorMetrics* out) {
   if (!h || !out) return SPH_ERR_INVALID_ARG;
   SPH_TRY(h, cudaSetDevice(h->dev));
-  double me[2] = {0.0, 0.0};
-  float var = 0.0f;
-  if (h->n > 0) {
-    enqueue_metrics(h);
-    SPH_TRY(h, cudaMemcpyAsync(me, h->me, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->st));
-    SPH_TRY(h, cudaMemcpyAsync(&var, h->var, sizeof(float), cudaMemcpyDeviceToHost, h->st));
-    SPH_TRY(h, cudaStreamSynchronize(h->st));
-  }
+  struct {
+    double me[2];
+    float var;
+    uint32_t flags;
+  } got{};  // as laid out at h->me
+  if (h->n > 0) enqueue_metrics(h);
+  else SPH_TRY(h, cudaMemsetAsync(h->me, 0, 2 * sizeof(double) + sizeof(float), h->st));
+  SPH_TRY(h, cudaMemcpyAsync(&got, h->me, sizeof got, cudaMemcpyDeviceToHost, h->st));
+  SPH_TRY(h, cudaStreamSynchronize(h->st));
+  const double* me = got.me;
+  const float var = got.var;
   double E0 = h->init_energy, M0 = h->init_mass;
   out->max_density_variation = var;
   out->energy_conservation = std::fabs(E0) > 1.0e-12 ? (float)std::fabs((me[1] - E0) / E0) : (float)std::fabs(me[1] - E0);
   out->mass_conservation = std::fabs(M0) > 1.0e-12 ? (float)std::fabs((me[0] - M0) / M0) : (float)std::fabs(me[0] - M0);
-  return check_device_flags(h);
+  return flags_status(h, got.flags);
 }
 
 size_t sph_particle_count(const SphHandle* h) { return h ? (size_t)h->n : 0; }
@@ -1999,9 +2174,7 @@ int sph_batch_timesteps(SphHandle* h, float* dt_out) {
   if (h->n == 0) return SPH_ERR_INVALID_ARG;
   ensure_red(h);
   enqueue_dt_finalize(h, h->dt_query);
-  SPH_TRY(h, cudaMemcpyAsync(dt_out, h->dt_query, sizeof(float) * h->ninst, cudaMemcpyDeviceToHost, h->st));
-  SPH_TRY(h, cudaStreamSynchronize(h->st));
-  return check_device_flags(h);
+  return read_dt(h, true, h->ninst, dt_out);
 }
 
 int sph_set_launch(SphHandle* h, const SphLaunch* l) {

@@ -372,7 +372,7 @@ class CudaKernel(SimulationKernel):
 
     def particles(self) -> ParticleArrays:
         if self._cache is None:
-            p = ParticleArrays.empty(self._n)
+            p = ParticleArrays.uninitialised(self._n)
             out = SphParticlesMut(self._n, *[_fp(getattr(p, f)) for f in PARTICLE_FIELDS],
                                   p.fluid_type.ctypes.data_as(_U8P))
             self._check(self._lib.sph_read_particles(self._h, C.byref(out)), "sph_read_particles")

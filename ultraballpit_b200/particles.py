@@ -60,6 +60,14 @@ class ParticleArrays:
         return p
 
     @classmethod
+    def uninitialised(cls, n: int) -> "ParticleArrays":
+        """Arrays for a read that fills them all: numpy backs large ones with huge pages, which a zeroed
+        allocation does not get, and first touches are most of a large read's time."""
+        p = cls(**{f: np.empty(n, dtype=np.float32) for f in PARTICLE_FIELDS})
+        p.fluid_type = np.empty(n, dtype=np.uint8)
+        return p
+
+    @classmethod
     def from_positions(cls, x, y, z, mass, density=1000.0, temperature=293.15,
                        fluid_type: FluidType = FluidType.Water) -> "ParticleArrays":
         """Vectorised ``push_particle`` (``particle.rs:96-120``): zero v, a, p."""
