@@ -203,101 +203,45 @@ __device__ __forceinline__ void colsum(float c[4], float& s0, float& s1) {
   }
 }
 
-// Backward pass of one tile given dy[16][16] (BF16, dL/dy in columns 0..3):
-// adds dL/dparams of the tile to gsum[kParams] (FP32, shared).
-__device__ __forceinline__ void backward_tile(const __nv_bfloat16* x, const __nv_bfloat16* w2,
-                                              const __nv_bfloat16* w3, const float* z1, const __nv_bfloat16* h1,
-                                              const float* z2, const __nv_bfloat16* h2, const __nv_bfloat16* dy,
-                                              __nv_bfloat16* dz, float* gsum, int lane) {
-  int g = lane >> 2, t = lane & 3;
-  // dW3[o][k] = sum_m dy[m][o] h2[m][k] (rows o >= 4 are padding)
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    mma_tile(dy, 1, 16, h2 + nt * 8, 64, 1, c, lane);
-    if (g < 4) {
-      gsum[kOffW3 + g * 64 + nt * 8 + 2 * t] += c[0];
-      gsum[kOffW3 + g * 64 + nt * 8 + 2 * t + 1] += c[1];
-    }
-  }
-  // db3
-  if (lane < 4) {
-    float s = 0.0f;
-    for (int m = 0; m < 16; ++m) s += __bfloat162float(dy[m * 16 + lane]);
-    gsum[kOffB3 + lane] += s;
-  }
-  // dz2 = (dy W3) * silu'(z2); db2
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    mma_tile(dy, 16, 1, w3 + nt * 8, 64, 1, c, lane);
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      int r = g + (e >> 1) * 8, col = nt * 8 + 2 * t + (e & 1);
-      c[e] *= silu_grad(z2[r * 64 + col]);
-      dz[r * 64 + col] = __float2bfloat16_rn(c[e]);
-    }
-    float s0, s1;
-    colsum(c, s0, s1);
-    if (lane < 4) {
-      gsum[kOffB2 + nt * 8 + 2 * t] += s0;
-      gsum[kOffB2 + nt * 8 + 2 * t + 1] += s1;
-    }
-  }
-  __syncwarp();
-  // dW2[o][k] = sum_m dz2[m][o] h1[m][k]
-#pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      mma_tile(dz + mt * 16, 1, 64, h1 + nt * 8, 64, 1, c, lane);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        int o = mt * 16 + g + (e >> 1) * 8, k = nt * 8 + 2 * t + (e & 1);
-        gsum[kOffW2 + o * 64 + k] += c[e];
-      }
-    }
-  // dz1 = (dz2 W2) * silu'(z1) (all tiles first: dz is overwritten after)
-  float d1[8][4];
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) d1[nt][e] = 0.0f;
-#pragma unroll
-    for (int kt = 0; kt < 4; ++kt) mma_tile(dz + kt * 16, 64, 1, w2 + kt * 16 * 64 + nt * 8, 64, 1, d1[nt], lane);
-  }
-  __syncwarp();
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      int r = g + (e >> 1) * 8, col = nt * 8 + 2 * t + (e & 1);
-      d1[nt][e] *= silu_grad(z1[r * 64 + col]);
-      dz[r * 64 + col] = __float2bfloat16_rn(d1[nt][e]);
-    }
-    float s0, s1;
-    colsum(d1[nt], s0, s1);
-    if (lane < 4) {
-      gsum[kOffB1 + nt * 8 + 2 * t] += s0;
-      gsum[kOffB1 + nt * 8 + 2 * t + 1] += s1;
-    }
-  }
-  __syncwarp();
-  // dW1[o][k] = sum_m dz1[m][o] x[m][k]
-#pragma unroll
-  for (int mt = 0; mt < 4; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 2; ++nt) {
-      float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      mma_tile(dz + mt * 16, 1, 64, x + nt * 8, 16, 1, c, lane);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        int o = mt * 16 + g + (e >> 1) * 8, k = nt * 8 + 2 * t + (e & 1);
-        gsum[kOffW1 + o * 16 + k] += c[e];
-      }
-    }
-  __syncwarp();
+// Fragments by ldmatrix: four (two) 8x8 BF16 matrices of a row-major array
+// in shared memory, each lane naming the 16-byte row it provides. Rows are
+// padded so that eight of them fall into distinct banks.
+constexpr int kPad16 = 24, kPad64 = 72;  // row strides of 16- and 64-wide arrays
+__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void ldm4(uint32_t r[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
+}
+__device__ __forceinline__ void ldm4t(uint32_t r[4], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)));
+}
+__device__ __forceinline__ void ldm2(uint32_t r[2], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1]) : "r"(smem_addr(p)));
+}
+__device__ __forceinline__ void ldm2t(uint32_t r[2], const __nv_bfloat16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];"
+               : "=r"(r[0]), "=r"(r[1]) : "r"(smem_addr(p)));
+}
+// A(16x16) of M[row][col] at (0, col): rows the samples
+__device__ __forceinline__ void frag_a(uint32_t a[4], const __nv_bfloat16* M, int ld, int col, int lane) {
+  ldm4(a, M + (lane & 15) * ld + col + (lane >> 4) * 8);
+}
+// A = M^T for M[k][m] at column m (k the 16 samples)
+__device__ __forceinline__ void frag_at(uint32_t a[4], const __nv_bfloat16* M, int ld, int m, int lane) {
+  ldm4t(a, M + ((lane & 7) + ((lane >> 4) & 1) * 8) * ld + m + ((lane >> 3) & 1) * 8);
+}
+// B(16x8) of W[n][k] at (n, k): the layer's weights
+__device__ __forceinline__ void frag_b(uint32_t b[2], const __nv_bfloat16* W, int ld, int n, int k, int lane) {
+  ldm2(b, W + (n + (lane & 7)) * ld + k + ((lane >> 3) & 1) * 8);
+}
+// B of M[k][n] at (k, n)
+__device__ __forceinline__ void frag_bt(uint32_t b[2], const __nv_bfloat16* M, int ld, int k, int n, int lane) {
+  ldm2t(b, M + (k + (lane & 15)) * ld + n);
+}
+__device__ __forceinline__ void mma_frag(float c[4], const uint32_t a[4], const uint32_t b[2]) {
+  mma_regs(c, a[0], a[1], a[2], a[3], b[0], b[1]);
 }
 
 }  // namespace sphmlp
