@@ -25,10 +25,11 @@
  *
  * Environment variables read at creation: SPH_TRACE (any value) prints the
  * creation's phase times on stderr; SPH_WARP_SCAN_MIN (a count) replaces the
- * size from which the density pass takes its warp-cooperative scan (384
- * particles per SM; 0 = always), and SPH_GROUP_LANES (1, 8 or 16) sets the
- * lanes that share a particle in the neighbour kernels, which otherwise follow
- * from the size. All forms give the same results bit for bit.
+ * size from which the density pass takes its warp-cooperative scan of 32
+ * particles a warp (1300 particles per SM; 0 = always), and SPH_GROUP_LANES (1,
+ * 8 or 16, or 2 for the density pass) sets the lanes that share a particle in
+ * the neighbour kernels, which otherwise follow from the size. All forms give
+ * the same results bit for bit.
  */
 #ifndef SPH_CUDA_H
 #define SPH_CUDA_H

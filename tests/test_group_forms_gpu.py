@@ -1,4 +1,4 @@
-"""The neighbour kernels with 1, 8 and 16 lanes per particle (SPH_GROUP_LANES)
+"""The neighbour kernels with 1, 2, 8 and 16 lanes per particle (SPH_GROUP_LANES)
 on the same cases, bit for bit against the oracle: sizes around a warp's and a
 block's particles, particles without neighbours, neighbourhoods past the masks
 and the list, corners whose boundary particles pass a group's shared terms,
@@ -17,7 +17,7 @@ from test_parity_gpu import assert_same, small_dam_break
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(params=["1", "8", "16"])
+@pytest.fixture(params=["1", "2", "8", "16"])
 def lanes(request, monkeypatch):
     monkeypatch.setenv("SPH_GROUP_LANES", request.param)
     return int(request.param)
@@ -43,7 +43,7 @@ def run(sc, order=CELL_ORDER_ROWS, steps=3, dt=2e-5):
 
 
 @pytest.mark.parametrize("order", [CELL_ORDER_ROWS, CELL_ORDER_MORTON])
-@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 8, 9, 31, 33, 129, 1000])
+@pytest.mark.parametrize("n", [1, 2, 3, 4, 5, 8, 9, 15, 16, 17, 31, 33, 129, 1000])
 def test_sizes(lanes, n, order):
     run(first(small_dam_break(), n), order)
 

@@ -614,21 +614,23 @@ void launch(SphHandle* h, void (*kernel)(P...), int grid, int block, size_t smem
 
 sph::Planes planes(SphHandle* h) { return sph::Planes{h->xyz, h->xyz_stride}; }
 
-// Lanes per particle by size, measured on B200 (the table in sph_group.cuh).
+// Lanes per particle by size, measured on B200 (the tables in sph_group.cuh).
 // The environment variable SPH_WARP_SCAN_MIN, read at creation, replaces the
-// count from which the density pass takes the warp-cooperative scan, and
-// SPH_GROUP_LANES (1, 8 or 16) sets the lanes of all three kernels.
+// count from which the density pass takes the warp-cooperative scan with 32
+// particles a warp, and SPH_GROUP_LANES sets the lanes of all three kernels (2:
+// of the density pass).
 void choose_lanes(SphHandle* h, int sms) {
   const long long n = h->n, per = sms;
   const int few = n <= 56 * per ? 16 : 8;
-  long long density_max = 384 * per;
-  if (const char* v = std::getenv("SPH_WARP_SCAN_MIN")) density_max = std::atoll(v) - 1;
-  h->lanes_density = n <= density_max ? few : 1;
+  long long one = 1300 * per;
+  if (const char* v = std::getenv("SPH_WARP_SCAN_MIN")) one = std::atoll(v) - 1;
+  h->lanes_density = n > one ? 1 : n <= 240 * per ? few : 2;
   h->lanes_forces = n <= 256 * per ? few : 1;
   h->lanes_xsph = n <= 128 * per ? few : 1;
   if (const char* v = std::getenv("SPH_GROUP_LANES")) {
     const int lanes = std::atoi(v);
     if (lanes == 1 || lanes == 8 || lanes == 16) h->lanes_xsph = h->lanes_density = h->lanes_forces = lanes;
+    if (lanes == 2) h->lanes_density = 2;
   }
 }
 
@@ -683,7 +685,7 @@ void enqueue_density_only(SphHandle* h) {
   // tile per warp (the fused inference)
   const size_t smem = (bs / 32) * sizeof(ScanWarp);
   const size_t smem_cl = smem + (bs / 32) * kClTileWords * sizeof(uint32_t);
-  if (h->lanes_density > 1) {
+  if (h->lanes_density > 2) {
     dispatch(h, false, [&](auto kp) {
       with_lanes(h->lanes_density, [&](auto lanes) {
         using KPT = decltype(kp);
@@ -700,6 +702,21 @@ void enqueue_density_only(SphHandle* h) {
         else if (h->cl_mode) run(k_density_group<KPT, 1, G>, smem1);
         else run(k_density_group<KPT, 0, G>, smem0);
       });
+    });
+    return;
+  }
+  if (h->lanes_density == 2) {
+    dispatch(h, false, [&](auto kp) {
+      using KPT = decltype(kp);
+      const size_t bytes = (kGroupThreads / 32) * sizeof(ScanWarp);
+      auto run = [&](auto kernel, size_t smem) {
+        launch(h, kernel, grid_for(h->n, kGroupThreads / 32 * kPairParticles), kGroupThreads, smem, kp, h->n, h->dt,
+               h->pos, planes(h), h->rv, h->id, h->ctab, h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
+               h->nbr, h->ncount, h->sdf, h->wall_tab, cb, h->slow);
+      };
+      if (h->cl_mode == 2) run(k_density_pair<KPT, 2>, bytes + (kGroupThreads / 32) * kClTileWords * sizeof(uint32_t));
+      else if (h->cl_mode) run(k_density_pair<KPT, 1>, bytes);
+      else run(k_density_pair<KPT, 0>, bytes);
     });
     return;
   }

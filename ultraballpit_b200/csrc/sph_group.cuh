@@ -18,7 +18,8 @@
 //    72,963    119 | 131               49 | 68              31 | 53
 // (the warp-cooperative density scan, 32 particles a warp: 113 at 72,963).
 // Hence 16 lanes up to 56 particles per SM, 8 above, for density and forces up
-// to 384 and 256 per SM, for XSPH up to 128.
+// to 240 and 256 per SM, for XSPH up to 128; density then takes two lanes per
+// particle (k_density_pair) up to 1300 per SM.
 #pragma once
 #include "sph_kernels.cuh"
 
@@ -432,6 +433,234 @@ k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __res
   }
   if (CL == 2) {
     uint32_t* tile = reinterpret_cast<uint32_t*>(s_dyn + (kGroupThreads / 32) * sizeof(SW)) + warp * kClTileWords;
+    network_epilogue(kp, i, near_wall, f, rho_pre, tile, id, rf, pr, cb, slow);
+  }
+}
+
+// Between the group form's sizes and those whose warps of 32 particles fill
+// the GPU: 16 particles a warp, two lanes each. The scan is scan_warp's with
+// 16 particles; in a round the pair's lanes take two neighbours each (entries
+// 4r, 4r + 1 and 4r + 2, 4r + 3 of the list), and the first adds its own terms,
+// then the other's. It executes 38 % more instructions than 32 particles a warp
+// and halves the chain. Density, us, 8 lanes | pair | 32 particles a warp:
+//   31k 66 | 66 | 103   50k 96 | 79 | 104   73k 131 | 95 | 111
+//   146k - | 166 | 178   250k - | 251 | 241   (69k without walls - | 87 | 106)
+// Eight blocks per SM at 64 registers; with six or five, 73k takes 113 or 117.
+constexpr int kPairParticles = 16;
+constexpr int kPairBlocks = 8;
+template <class KP, int CL>
+__global__ void __launch_bounds__(kGroupThreads, kPairBlocks)
+k_density_pair(KP kp, int n, const float* __restrict__ dtp, const float4* __restrict__ pos, Planes pl,
+               const float2* __restrict__ rv, const uint32_t* __restrict__ id, const uint2* __restrict__ ctab,
+               const uint32_t* __restrict__ bc_start, const uint32_t* __restrict__ bc_list,
+               const float4* __restrict__ bpos, float2* __restrict__ rf, float* __restrict__ pr,
+               const uint32_t* __restrict__ err, uint32_t* __restrict__ nbr, uint32_t* __restrict__ ncount,
+               const float* __restrict__ sdf, const float2* __restrict__ wall_tab, ClosureBufs cb,
+               uint32_t* __restrict__ slow) {
+  constexpr unsigned kAll = 0xffffffffu;
+  constexpr int P = kPairParticles;
+  extern __shared__ __align__(16) unsigned char s_dyn[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  ScanWarp& S = reinterpret_cast<ScanWarp*>(s_dyn)[warp];
+  const int base = (int)((blockIdx.x * kGroupThreads + threadIdx.x) >> 5) * P;
+  if (base >= n || *err) return;  // whole warps
+  const int p = lane & (P - 1);
+  const bool second = lane >= P;
+  const bool live = base + p < n;
+  const int i = live ? base + p : base;
+  const SimConst& k = kp.at(i);
+  const float4 pi = pos[i];
+  const float rho_old_i = rv[i].x;
+  const bool delta = (k.flags & kFlagDelta) != 0;
+  const int cx = axis_cell(pi.x, k.gmin[0], k.cell, k.dims[0]);
+  const int cy = axis_cell(pi.y, k.gmin[1], k.cell, k.dims[1]);
+  const int cz = axis_cell(pi.z, k.gmin[2], k.cell, k.dims[2]);
+  const int lin = cell_hash(cx, cy, cz, k);
+  const uint32_t gkey = (uint32_t)(k.coff + lin);
+  const uint32_t gprev = __shfl_up_sync(kAll, gkey, 1);
+  const uint32_t heads = __ballot_sync(kAll, live && !second && (lane == 0 || gprev != gkey));
+  const int nlive = min(P, n - base);
+  const int myhead = 31 - __clz(heads & ((2u << p) - 1u));
+  const uint32_t hmask = 1u << myhead;
+  float rho = pi.w * k.norm_h3, diff_sum = 0.0f, ssum = 0.0f;  // the first lane's
+  uint32_t key = 0xffffffffu, mine = 0;  // mine: the neighbours this lane takes
+  float dmin = INFINITY;
+  bool fed = true;
+  uint32_t dense = 0;  // neighbours of a particle whose neighbourhood passes the masks
+  uint32_t rem = heads;
+  while (rem) {
+    uint32_t batch = 0, t = rem;  // the next kScanSegs segments
+    for (int q = 0; q < kScanSegs && t; ++q) {
+      batch |= t & (0u - t);
+      t &= t - 1u;
+    }
+    rem = t;
+    __syncwarp();
+    int seg = 0;
+    uint32_t mbase = 0;
+    for (uint32_t bb = batch; bb; bb &= bb - 1u, ++seg) {
+      const int hl = __ffs(bb) - 1;
+      const uint32_t after = heads & ~((2u << hl) - 1u);
+      const int he = after ? __ffs(after) - 1 : nlive;
+      const int sx = __shfl_sync(kAll, cx, hl), sy = __shfl_sync(kAll, cy, hl), sz = __shfl_sync(kAll, cz, hl);
+      const SimConst& ks = kp.at(__shfl_sync(kAll, i, hl));
+      const int nw = scan_segment(S, seg, hl, he, mbase, ks, sx, sy, sz, pi.x, pi.y, pi.z, pl, ctab);
+      if (nw <= kScanWords) mbase += (uint32_t)(nw * ((he - hl + 3) & ~3));
+      __syncwarp();
+    }
+    const bool in_batch = live && (batch & hmask);
+    const int s = __popc(batch & (hmask - 1u));
+    const int R = k.rows ? 9 : 27;
+    const uint32_t total = in_batch ? S.vstart[s][R] : 0u;
+    const int nw = (int)((total + 31u) / 32u);
+    const bool act = in_batch && nw <= kScanWords;
+    if (in_batch && !act) {
+      fed = false;
+      if (!second) dense = record_neighbors(pi.x, pi.y, pi.z, i, pl, ctab, ScanGeo(k), nbr, n);
+    }
+    __syncwarp();
+    const uint32_t q4 = act ? S.mquad[s] : 0u;
+    const uint32_t* words = S.mask + (act ? S.mbase[s] + (uint32_t)(p - myhead) : 0u);
+    const uint32_t vself = act ? S.vstart[s][R / 2] + ((uint32_t)i - S.sstart[s][R / 2]) : 0u;
+    const int wself = act ? (int)(vself >> 5) : -1;
+    const uint32_t bself = ~(1u << (vself & 31u));
+    int w = 0, r = 0;
+    uint32_t M = act ? words[0] : 0u;
+    if (wself == 0) M &= bself;
+    uint32_t vnext = act ? S.vstart[s][1] : 0u;
+    uint32_t off = act ? S.sstart[s][0] - S.vstart[s][0] : 0u;
+    auto more = [&] {  // the next set bit's word, if any is left
+      while (M == 0u && w + 1 < nw) {
+        M = words[++w * q4];
+        if (w == wself) M &= bself;
+      }
+      return M != 0u;
+    };
+    auto next = [&](uint32_t& slot) {
+      if (!act || !more()) return false;
+      const uint32_t v = (uint32_t)(w * 32 + __ffs(M) - 1);
+      M &= M - 1u;
+      while (v >= vnext) {
+        ++r;
+        vnext = S.vstart[s][r + 1];
+        off = S.sstart[s][r] - S.vstart[s][r];
+      }
+      slot = v + off;
+      ++mine;
+      return true;
+    };
+    auto skip2 = [&] {
+      if (act && more()) {
+        M &= M - 1u;
+        if (more()) M &= M - 1u;
+      }
+    };
+    if (second) skip2();
+    uint2* at = reinterpret_cast<uint2*>(reinterpret_cast<uint4*>(nbr) + i) + (second ? 1 : 0);
+    for (uint32_t q = 0;; ++q, at += 2 * (size_t)n) {
+      uint32_t sa = (uint32_t)i, sb = (uint32_t)i;
+      const bool g0 = next(sa), g1 = g0 && next(sb);
+      if (!__any_sync(kAll, g0)) break;
+      const float4 p0 = __ldg(&pos[sa]), p1 = __ldg(&pos[sb]);
+      const float2 r0 = __ldg(&rv[sa]), r1 = __ldg(&rv[sb]);
+      auto term = [&](bool in, const float4& pj, const float2& rvj, float& a, float& d, float& v) {
+        const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+        const float d2 = in ? dx * dx + dy * dy + dz * dz : 1.0f;
+        float wt, half_diff;
+        if (delta) density_fast<true>(k, pj.w, rvj, rho_old_i, dx, dy, dz, d2, key, dmin, wt, half_diff);
+        else density_fast<false>(k, pj.w, rvj, rho_old_i, dx, dy, dz, d2, key, dmin, wt, half_diff);
+        a = in ? pj.w * wt : 0.0f;
+        d = in ? 2.0f * half_diff : 0.0f;
+        v = CL && in ? rvj.y * wt : 0.0f;
+      };
+      float a0, a1, d0, d1, v0, v1;
+      term(g0, p0, r0, a0, d0, v0);
+      term(g1, p1, r1, a1, d1, v1);
+      if (g0 && q < kNbrCap / 4) *at = make_uint2(sa, sb);
+      const float b0 = __shfl_down_sync(kAll, a0, P), b1 = __shfl_down_sync(kAll, a1, P);
+      const float e0 = __shfl_down_sync(kAll, d0, P), e1 = __shfl_down_sync(kAll, d1, P);
+      rho += a0;
+      rho += a1;
+      rho += b0;
+      rho += b1;
+      diff_sum += d0;
+      diff_sum += d1;
+      diff_sum += e0;
+      diff_sum += e1;
+      if (CL) {
+        const float f0 = __shfl_down_sync(kAll, v0, P), f1 = __shfl_down_sync(kAll, v1, P);
+        ssum += v0;
+        ssum += v1;
+        ssum += f0;
+        ssum += f1;
+      }
+      skip2();
+    }
+    __syncwarp();
+  }
+  const uint32_t listed = __shfl_sync(kAll, dense, p) + mine + __shfl_xor_sync(kAll, mine, P);
+  key = min(key, __shfl_xor_sync(kAll, key, P));
+  dmin = fminf(dmin, __shfl_xor_sync(kAll, dmin, P));
+  const bool close = dmin < kTinyD2;
+  if (live && !second && (!fed || !k.fast || close || key < k.diff_key || !finite3(rho, diff_sum, 0.0f))) {
+    const DensitySum e = density_exact(kp.ref(i), i, pi, rho_old_i, pos, rv, ctab);
+    rho = e.rho;
+    diff_sum = e.diff;
+    if (CL) ssum = e.ssum;
+  }
+  __syncwarp();
+  // boundary terms, four candidates a round, two a lane; those in support
+  // follow the neighbours in the list
+  float rho_wall = 0.0f;
+  uint32_t nwall = 0;
+  const uint32_t q0 = live ? __ldg(&bc_start[k.coff + lin]) : 0u, q1 = live ? __ldg(&bc_start[k.coff + lin + 1]) : 0u;
+  const uint32_t mine0 = min(q0 + (second ? 2u : 0u), q1);
+  BoundaryWalk<2> walk(q0 < q1 ? mine0 : 0u, q0 < q1 ? q1 : 0u, bc_list, bpos, 4u);
+  for (uint32_t q = q0; __any_sync(kAll, q < q1); q += 4) {
+    const uint32_t qa = q + (second ? 2u : 0u);
+    const bool va = qa < q1, vb = qa + 1 < q1;
+    uint32_t bi[2] = {0u, 0u};
+    float4 bp[2] = {make_float4(0.0f, 0.0f, 0.0f, 0.0f), make_float4(0.0f, 0.0f, 0.0f, 0.0f)};
+    if (va) walk.round(qa, bi, bp);
+    const uint32_t ia = bi[0], ib = bi[1];
+    const float4 ba = bp[0], bb = bp[1];
+    auto d2_of = [&](const float4& b) {
+      const float dx = pi.x - b.x, dy = pi.y - b.y, dz = pi.z - b.z;
+      return dx * dx + dy * dy + dz * dz;
+    };
+    const float da = d2_of(ba), db = d2_of(bb);
+    const bool ina = va && da <= k.sup_d2, inb = vb && db <= k.sup_d2;
+    const uint32_t ma = __ballot_sync(kAll, ina), mb = __ballot_sync(kAll, inb);
+    if ((ma | mb) == 0u) continue;
+    const float wa = ina ? ba.w * w_c2(sqrt_any(da), k) : 0.0f, wb = inb ? bb.w * w_c2(sqrt_any(db), k) : 0.0f;
+    const float xa = __shfl_down_sync(kAll, wa, P), xb = __shfl_down_sync(kAll, wb, P);
+    rho += wa;
+    rho += wb;
+    rho += xa;
+    rho += xb;
+    if (CL) {
+      rho_wall += wa;
+      rho_wall += wb;
+      rho_wall += xa;
+      rho_wall += xb;
+    }
+    const uint32_t first = ((ma >> p) & 1u) + ((mb >> p) & 1u);  // the first lane's
+    uint32_t e = listed + nwall + (second ? first : 0u);
+    if (ina && e < kNbrCap) nbr[nbr_index(e, n, i)] = ia;
+    e += ina ? 1u : 0u;
+    if (inb && e < kNbrCap) nbr[nbr_index(e, n, i)] = ib;
+    nwall += first + ((ma >> (p + P)) & 1u) + ((mb >> (p + P)) & 1u);
+  }
+  float f[16];
+  float rho_pre = 0.0f;
+  bool near_wall = false;
+  if (live && !second) {
+    ncount[i] = pack_counts(listed, nwall, close);
+    near_wall = density_finish<CL>(k, i, dtp[k.inst], pi, DensityState{rho, diff_sum, ssum, rho_wall, nwall, listed},
+                                   rv, id, rf, pr, sdf, wall_tab, cb, slow, f, rho_pre);
+  }
+  if (CL == 2) {
+    uint32_t* tile = reinterpret_cast<uint32_t*>(s_dyn + (kGroupThreads / 32) * sizeof(ScanWarp)) + warp * kClTileWords;
     network_epilogue(kp, i, near_wall, f, rho_pre, tile, id, rf, pr, cb, slow);
   }
 }
