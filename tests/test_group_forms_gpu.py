@@ -117,3 +117,25 @@ def test_closure_and_sdf_walls_equal_the_thread_form(lanes, mode, monkeypatch):
         assert_same(a[0], b[0])
         for x, y in zip(a[1:], b[1:]):
             np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [1, 3, 15, 16, 17, 63, 115])
+def test_closure_at_a_tile_s_and_a_block_s_edges(lanes, n, monkeypatch):
+    """A tile of the network holds 16 particles; a block of the group forms' 8
+    or 16 shares one, whatever part of them is there and near the wall."""
+    out = []
+    for form in (str(lanes), "1"):
+        monkeypatch.setenv("SPH_GROUP_LANES", form)
+        sc = first(domain.tank_with_sphere(0.004, domain_max=(0.02, 0.02, 0.03), center=(0.01, 0.01, 0.008),
+                                           radius=0.005, fill_height=0.018, geometry="lattice"), n)
+        k = CudaKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta)
+        k.set_feature_sdf(sc.sdf)
+        k.set_closure(2, ClosureNet(seed=4).params())
+        k.step_auto(2)
+        ids, feat, rho = k.closure_samples()
+        o = np.argsort(ids)
+        out.append((k.particles(), ids[o], feat[o], rho[o]))
+        k.close()
+    assert_same(out[0][0], out[1][0])
+    for x, y in zip(out[0][1:], out[1][1:]):
+        np.testing.assert_array_equal(x, y)

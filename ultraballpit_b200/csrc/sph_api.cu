@@ -124,7 +124,7 @@ struct SphHandle {
   uint32_t *cl_count = nullptr, *cl_slot = nullptr;
   float *cl_feat = nullptr, *cl_rho = nullptr, *cl_wf = nullptr;
   float4* corr = nullptr;
-  __nv_bfloat16* cl_wb = nullptr;
+  uint4* cl_wq = nullptr;
   // scalars, one allocation so that one copy reads a result with the error
   // flags: (mass, energy) sums, density variation, flags, the step's dt and
   // the queried one per instance
@@ -679,7 +679,7 @@ void enqueue_scan_fill(SphHandle* h) {
 void enqueue_density_only(SphHandle* h) {
   using namespace sph;
   int bs = h->bs_density;
-  sph::ClosureBufs cb{h->cl_count, h->cl_slot, h->cl_feat, h->cl_rho, h->corr, h->vel, h->cl_wb, h->cl_wf};
+  sph::ClosureBufs cb{h->cl_count, h->cl_slot, h->cl_feat, h->cl_rho, h->corr, h->vel, h->cl_wq, h->cl_wf};
   if (h->cl_mode) cudaMemsetAsync(h->cl_count, 0, sizeof(uint32_t), h->st);
   // the warp scan's scratch per warp; closure mode 2 adds a 16-sample network
   // tile per warp (the fused inference)
@@ -698,7 +698,7 @@ void enqueue_density_only(SphHandle* h) {
                  h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
                  h->slow);
         };
-        if (h->cl_mode == 2) run(k_density_group<KPT, 2, G>, smem1 + (kGroupThreads / 32) * kClTileWords * sizeof(uint32_t));
+        if (h->cl_mode == 2) run(k_density_group<KPT, 2, G>, smem1 + sizeof(BlockTile));
         else if (h->cl_mode) run(k_density_group<KPT, 1, G>, smem1);
         else run(k_density_group<KPT, 0, G>, smem0);
       });
@@ -2341,7 +2341,7 @@ int sph_set_closure(SphHandle* h, int mode, const float* params) {
     if (e == cudaSuccess) e = dalloc(h, &h->cl_rho, n);
     if (e == cudaSuccess) e = dalloc(h, &h->corr, n);
     if (e == cudaSuccess) e = dalloc(h, &h->cl_wf, sphmlp::kParams);
-    if (e == cudaSuccess) e = dalloc(h, &h->cl_wb, sphmlp::kBf16Count);
+    if (e == cudaSuccess) e = dalloc(h, &h->cl_wq, sphmlp::kFragQuads * 32);
     if (e != cudaSuccess) return cuda_status(h, e, "closure allocation");
     SPH_TRY(h, cudaMemsetAsync(h->cl_count, 0, sizeof(uint32_t), h->st));
     SPH_TRY(h, cudaMemsetAsync(h->corr, 0, std::max<size_t>(n, 1) * sizeof(float4), h->st));
@@ -2353,8 +2353,12 @@ int sph_set_closure(SphHandle* h, int mode, const float* params) {
       if (bi >= 0) wb[bi] = __float2bfloat16_rn(params[i]);
     }
     SPH_TRY(h, cudaMemcpyAsync(h->cl_wf, params, sphmlp::kParams * sizeof(float), cudaMemcpyHostToDevice, h->st));
-    SPH_TRY(h, cudaMemcpyAsync(h->cl_wb, wb.data(), wb.size() * sizeof(__nv_bfloat16), cudaMemcpyHostToDevice,
-                               h->st));
+    std::vector<uint32_t> frag(sphmlp::kFragWords, 0u);
+    for (int at = 0; at < sphmlp::kFragWords; ++at) {
+      const int bi = sphmlp::frag_index(at);
+      if (bi >= 0) memcpy(&frag[at], &wb[bi], sizeof(uint32_t));
+    }
+    SPH_TRY(h, cudaMemcpyAsync(h->cl_wq, frag.data(), frag.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, h->st));
     SPH_TRY(h, cudaStreamSynchronize(h->st));
   }
   h->cl_mode = mode;

@@ -222,6 +222,41 @@ struct __align__(16) CoopWarp {
   uint32_t mbase[kPad], mquad[kPad];
 };
 
+// The closure's feature probes (feature_probe) of a particle held by L lanes,
+// `sub` this one's number and get(v, l) lane l's v: each lane reads its share
+// and every lane ends up with all twelve. Every lane of the warp takes part,
+// `near` if its particle is near the wall. Bound by latency: one lane alone
+// read them in turn, some 100 gathers and 36 divisions, and they took 22 of
+// the 107 us of a 24k-particle tank's density pass; shared by 8 lanes they
+// take 6, by the pair form's 2 some 6 of 133 us at 42k particles.
+template <int L, class Get>
+__device__ __forceinline__ void share_probes(const SimConst& k, const float* __restrict__ sdf, const float4& pi,
+                                             int sub, bool near, float centre, Get get, float out[12]) {
+  if (!__any_sync(0xffffffffu, near)) return;
+  const bool grad = near && wall_is_sdf(k, pi, centre);
+  constexpr int R = (12 + L - 1) / L;
+  float own[R];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int a = r * L + sub;
+    own[r] = a < 12 && (a < 6 ? grad : near) ? feature_probe(k, sdf, pi, a) : 0.0f;
+  }
+#pragma unroll
+  for (int a = 0; a < 12; ++a) out[a] = get(own[a / L], a % L);
+}
+
+// The closure network's tile of a block in the group form: a row per
+// particle, taken by the block's last warp to arrive, which nobody waits for.
+// A tile a warp was 4 rows of 16 with 8 lanes a particle: the network took 27
+// us of the same pass, and takes 14 with one tile a block. The two together:
+// 45 -> 37 / 63 -> 55 / 107 -> 86 us at 5k / 13k / 24k particles.
+struct BlockTile {
+  uint32_t xy[kClTileWords];  // network_epilogue's tile
+  int owner[16];              // the row's particle, -1 for none
+  float rho_pre[16];
+  uint32_t arrived;           // warps, and (from bit 16 up) their particles near the wall
+};
+
 template <class KP, int CL, int G>
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
 k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __restrict__ pos, Planes pl,
@@ -237,8 +272,15 @@ k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __res
   using SW = CoopWarp<G, NC>;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   SW& S = reinterpret_cast<SW*>(s_dyn)[warp];
+  BlockTile& B = *reinterpret_cast<BlockTile*>(s_dyn + (kGroupThreads / 32) * sizeof(SW));  // CL == 2
   const Group<G> g;
   const int base = (int)((blockIdx.x * kGroupThreads + threadIdx.x) >> 5) * P;
+  if (CL == 2) {
+    B.xy[threadIdx.x] = 0u;  // the x tile: 128 words
+    if (threadIdx.x < 16) B.owner[threadIdx.x] = -1;
+    if (threadIdx.x == 0) B.arrived = 0u;
+    __syncthreads();
+  }
   if (base >= n || *err) return;  // whole warps
   const int mine_p = lane / G;    // the group's particle within the warp
   const bool live = base + mine_p < n;
@@ -424,16 +466,44 @@ k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __res
   }
   rho = g.get(wsum, 0);
   const DensityState st{rho, diff_sum, ssum, CL ? g.get(wsum, 1) : 0.0f, nwall, listed};
+  const float centre = live ? centre_sdf<CL>(k, sdf, pi) : 0.0f;
+  float probes[CL ? 12 : 1];
+  if (CL)
+    share_probes<G>(k, sdf, pi, g.sub, live && k.feat_sdf && centre_feature(k, pi, centre) < k.support, centre,
+                    [&](float v, int l) { return g.get(v, l); }, probes);
   float f[16];
   float rho_pre = 0.0f;
   bool near_wall = false;
   if (live && g.sub == 0) {
     ncount[i] = pack_counts(listed, nwall, close);
-    near_wall = density_finish<CL>(k, i, dtp[k.inst], pi, st, rv, id, rf, pr, sdf, wall_tab, cb, slow, f, rho_pre);
+    near_wall = density_finish<CL>(k, i, dtp[k.inst], pi, st, rv, id, rf, pr, centre,
+                                   [&](int a) { return probes[CL ? a : 0]; }, wall_tab, cb, slow, f, rho_pre);
   }
   if (CL == 2) {
-    uint32_t* tile = reinterpret_cast<uint32_t*>(s_dyn + (kGroupThreads / 32) * sizeof(SW)) + warp * kClTileWords;
-    network_epilogue(kp, i, near_wall, f, rho_pre, tile, id, rf, pr, cb, slow);
+    constexpr int W = kGroupThreads / 32;
+    static_assert(W * P <= 16 && kGroupThreads == 16 * 16 / 2, "a block's particles are one tile");
+    __nv_bfloat16* xt = reinterpret_cast<__nv_bfloat16*>(B.xy);
+    float* yt = reinterpret_cast<float*>(B.xy + 16 * 16 / 2);
+    const int row = warp * P + mine_p;
+    if (near_wall) {
+#pragma unroll
+      for (int a = 0; a < 16; ++a) xt[row * 16 + a] = __float2bfloat16_rn(f[a]);
+      B.owner[row] = i;
+      B.rho_pre[row] = rho_pre;
+    }
+    const uint32_t rows = (uint32_t)__popc(__ballot_sync(kAll, near_wall));
+    // the rows, and density_finish's results, are there for the last to arrive
+    __threadfence_block();
+    __syncwarp();
+    const uint32_t before = __shfl_sync(kAll, lane == 0 ? atomicAdd(&B.arrived, 1u + (rows << 16)) : 0u, 0);
+    const int warps = min(W, (n - (base - warp * P) + P - 1) / P);
+    if ((int)(before & 0xffffu) != warps - 1 || (before >> 16) + rows == 0u) return;
+    __threadfence_block();
+    sphmlp::forward_tile_regs(xt, cb.wq, cb.wf, yt, lane);
+    __syncwarp();
+    const int o = lane < 16 ? B.owner[lane] : -1;
+    if (o >= 0)
+      closure_apply_one(kp.at(o), o, (id[o] & kAirBit) != 0, B.rho_pre[lane], yt + lane * 4, rf, pr, cb.corr, slow);
   }
 }
 
@@ -651,13 +721,19 @@ k_density_pair(KP kp, int n, const float* __restrict__ dtp, const float4* __rest
     if (inb && e < kNbrCap) nbr[nbr_index(e, n, i)] = ib;
     nwall += first + ((ma >> (p + P)) & 1u) + ((mb >> (p + P)) & 1u);
   }
+  const float centre = live ? centre_sdf<CL>(k, sdf, pi) : 0.0f;
+  float probes[CL ? 12 : 1];
+  if (CL)
+    share_probes<2>(k, sdf, pi, second ? 1 : 0, live && k.feat_sdf && centre_feature(k, pi, centre) < k.support, centre,
+                    [&](float v, int l) { return __shfl_sync(kAll, v, p + l * P); }, probes);
   float f[16];
   float rho_pre = 0.0f;
   bool near_wall = false;
   if (live && !second) {
     ncount[i] = pack_counts(listed, nwall, close);
     near_wall = density_finish<CL>(k, i, dtp[k.inst], pi, DensityState{rho, diff_sum, ssum, rho_wall, nwall, listed},
-                                   rv, id, rf, pr, sdf, wall_tab, cb, slow, f, rho_pre);
+                                   rv, id, rf, pr, centre, [&](int a) { return probes[CL ? a : 0]; }, wall_tab, cb,
+                                   slow, f, rho_pre);
   }
   if (CL == 2) {
     uint32_t* tile = reinterpret_cast<uint32_t*>(s_dyn + (kGroupThreads / 32) * sizeof(ScanWarp)) + warp * kClTileWords;

@@ -122,19 +122,34 @@ __device__ __forceinline__ void mma_regs(float c[4], uint32_t a0, uint32_t a1, u
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ uint32_t ldg_pair(const __nv_bfloat16* p) {
-  return __ldg(reinterpret_cast<const unsigned int*>(p));
+// The weights in the order the forward pass's lanes take them: per lane 22
+// quads of words, 4 of W1 (two n-tiles' B fragments each), 16 of W2 (two
+// k-tiles' each) and 2 of W3 (two k-tiles' each; its columns 4..7 are zero
+// rows), quad q of lane l at word (q * 32 + l) * 4. A quad is one coalesced
+// load; a word at a time from the row-major matrices is 72 loads of eight
+// lines each (density pass of a 42k-particle tank, two lanes a particle: 127
+// -> 123 us; 88 -> 86 at 24k).
+constexpr int kFragQuads = 22, kFragWords = kFragQuads * 32 * 4;
+
+// Word `at` of that array as the index of its lower BF16 in W1 | W2 | W3
+// (the upper one follows it), -1 for a zero.
+__host__ __device__ inline int frag_index(int at) {
+  const int e = at & 3, lane = (at >> 2) & 31, q = at >> 7;
+  const int g = lane >> 2, k0 = 2 * (lane & 3) + (e & 1) * 8, odd = e >> 1;
+  if (q < 4) return ((2 * q + odd) * 8 + g) * 16 + k0;
+  if (q < 20) return 1024 + (((q - 4) >> 1) * 8 + g) * 64 + (((q - 4) & 1) * 2 + odd) * 16 + k0;
+  return g < 4 ? 5120 + g * 64 + ((q - 20) * 2 + odd) * 16 + k0 : -1;
 }
 
 // The forward pass of forward_tile with the activations kept in registers:
 // the C fragment of two adjacent n-tiles of one layer is the A fragment of
 // one k-tile of the next (rows g, g+8; columns 2t, 2t+1 and 2t+8, 2t+9), so
 // only the input tile x[16][16] (BF16, shared) and the output y[16][4]
-// (FP32, shared) leave the registers. The weights are read from global
-// memory (wb: BF16 W1 | W2 | W3; the master FP32 parameters wf for the
+// (FP32, shared) leave the registers. The weights come from global memory in
+// the lanes' order (wq, frag_index; the master FP32 parameters wf for the
 // biases) and stay in L1. Same instructions, operands and rounding points as
 // forward_tile, so the outputs are identical.
-__device__ __forceinline__ void forward_tile_regs(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ wb,
+__device__ __forceinline__ void forward_tile_regs(const __nv_bfloat16* x, const uint4* __restrict__ wq,
                                                   const float* __restrict__ wf, float* y, int lane) {
   int g = lane >> 2, t = lane & 3;
   int k0 = 2 * t;
@@ -142,46 +157,40 @@ __device__ __forceinline__ void forward_tile_regs(const __nv_bfloat16* x, const 
   uint32_t xa1 = pack2(x[(g + 8) * 16 + k0], x[(g + 8) * 16 + k0 + 1]);
   uint32_t xa2 = pack2(x[g * 16 + k0 + 8], x[g * 16 + k0 + 9]);
   uint32_t xa3 = pack2(x[(g + 8) * 16 + k0 + 8], x[(g + 8) * 16 + k0 + 9]);
-  const __nv_bfloat16* w1 = wb;
-  const __nv_bfloat16* w2 = wb + 1024;
-  const __nv_bfloat16* w3 = wb + 5120;
-  uint32_t h1[16];
+  wq += lane;
+  uint32_t h1[16], h2[16];
+  // an n-tile's sums with their biases through the SiLU, as half an A fragment
+  auto activate = [&](const float c[4], int off, int nt, uint32_t* h) {
+    const float2 b = __ldg(reinterpret_cast<const float2*>(wf + off + nt * 8 + k0));
+    h[(nt >> 1) * 4 + (nt & 1) * 2] = pack2(__float2bfloat16_rn(silu(c[0] + b.x)), __float2bfloat16_rn(silu(c[1] + b.y)));
+    h[(nt >> 1) * 4 + (nt & 1) * 2 + 1] =
+        pack2(__float2bfloat16_rn(silu(c[2] + b.x)), __float2bfloat16_rn(silu(c[3] + b.y)));
+  };
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint4 w = __ldg(wq + q * 32);
+    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    mma_regs(c, xa0, xa1, xa2, xa3, w.x, w.y);
+    mma_regs(d, xa0, xa1, xa2, xa3, w.z, w.w);
+    activate(c, kOffB1, 2 * q, h1);
+    activate(d, kOffB1, 2 * q + 1, h1);
+  }
 #pragma unroll
   for (int nt = 0; nt < 8; ++nt) {
+    const uint4 u = __ldg(wq + (4 + 2 * nt) * 32), v = __ldg(wq + (5 + 2 * nt) * 32);
     float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    const __nv_bfloat16* wr = w1 + (nt * 8 + g) * 16 + k0;
-    mma_regs(c, xa0, xa1, xa2, xa3, ldg_pair(wr), ldg_pair(wr + 8));
-    float bl = __ldg(&wf[kOffB1 + nt * 8 + k0]), bh = __ldg(&wf[kOffB1 + nt * 8 + k0 + 1]);
-    h1[(nt >> 1) * 4 + (nt & 1) * 2] = pack2(__float2bfloat16_rn(silu(c[0] + bl)), __float2bfloat16_rn(silu(c[1] + bh)));
-    h1[(nt >> 1) * 4 + (nt & 1) * 2 + 1] =
-        pack2(__float2bfloat16_rn(silu(c[2] + bl)), __float2bfloat16_rn(silu(c[3] + bh)));
+    mma_regs(c, h1[0], h1[1], h1[2], h1[3], u.x, u.y);
+    mma_regs(c, h1[4], h1[5], h1[6], h1[7], u.z, u.w);
+    mma_regs(c, h1[8], h1[9], h1[10], h1[11], v.x, v.y);
+    mma_regs(c, h1[12], h1[13], h1[14], h1[15], v.z, v.w);
+    activate(c, kOffB2, nt, h2);
   }
-  uint32_t h2[16];
-#pragma unroll
-  for (int nt = 0; nt < 8; ++nt) {
-    float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int kt = 0; kt < 4; ++kt) {
-      const __nv_bfloat16* wr = w2 + (nt * 8 + g) * 64 + kt * 16 + k0;
-      mma_regs(c, h1[kt * 4], h1[kt * 4 + 1], h1[kt * 4 + 2], h1[kt * 4 + 3], ldg_pair(wr), ldg_pair(wr + 8));
-    }
-    float bl = __ldg(&wf[kOffB2 + nt * 8 + k0]), bh = __ldg(&wf[kOffB2 + nt * 8 + k0 + 1]);
-    h2[(nt >> 1) * 4 + (nt & 1) * 2] = pack2(__float2bfloat16_rn(silu(c[0] + bl)), __float2bfloat16_rn(silu(c[1] + bh)));
-    h2[(nt >> 1) * 4 + (nt & 1) * 2 + 1] =
-        pack2(__float2bfloat16_rn(silu(c[2] + bl)), __float2bfloat16_rn(silu(c[3] + bh)));
-  }
+  const uint4 u = __ldg(wq + 20 * 32), v = __ldg(wq + 21 * 32);
   float c[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-  for (int kt = 0; kt < 4; ++kt) {
-    // output columns 4..7 of the padded W3 are zero rows
-    uint32_t b0 = 0u, b1 = 0u;
-    if (g < 4) {
-      const __nv_bfloat16* wr = w3 + g * 64 + kt * 16 + k0;
-      b0 = ldg_pair(wr);
-      b1 = ldg_pair(wr + 8);
-    }
-    mma_regs(c, h2[kt * 4], h2[kt * 4 + 1], h2[kt * 4 + 2], h2[kt * 4 + 3], b0, b1);
-  }
+  mma_regs(c, h2[0], h2[1], h2[2], h2[3], u.x, u.y);
+  mma_regs(c, h2[4], h2[5], h2[6], h2[7], u.z, u.w);
+  mma_regs(c, h2[8], h2[9], h2[10], h2[11], v.x, v.y);
+  mma_regs(c, h2[12], h2[13], h2[14], h2[15], v.z, v.w);
   if (t < 2) {
     float bl = __ldg(&wf[kOffB3 + k0]), bh = __ldg(&wf[kOffB3 + k0 + 1]);
     y[g * 4 + k0] = c[0] + bl;
