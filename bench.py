@@ -89,7 +89,8 @@ def roofline_bytes():
     return {k: int(v) for k, v in re.findall(r"#define (SPH_\w+) (\d+)", src)}
 
 
-KERNEL_SOURCES = ["ultraballpit_b200/csrc/sph_kernels.cuh", "ultraballpit_b200/csrc/sph_mlp.cuh"]
+KERNEL_SOURCES = ["ultraballpit_b200/csrc/sph_kernels.cuh", "ultraballpit_b200/csrc/sph_group.cuh",
+                  "ultraballpit_b200/csrc/sph_mlp.cuh"]
 
 
 def strip_source(src: bytes) -> bytes:
