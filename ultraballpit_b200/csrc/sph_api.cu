@@ -107,7 +107,7 @@ struct SphHandle {
   // boundary
   float4* bpos = nullptr;
   float* bpress = nullptr;
-  // per boundary particle: the fluid particles in its support (k_wall_scatter;
+  // per boundary particle: the fluid particles in its support (scatter_walls;
   // wlist null where its memory could not be had: k_adami then searches)
   uint32_t *wcount = nullptr, *wlist = nullptr;
   int pool = -1;  // device arrays from the library's pool (1) or cudaMalloc (0); set by the first one
@@ -676,10 +676,13 @@ void enqueue_scan_fill(SphHandle* h) {
   launch(h, k_fill, grid_for(h->n, 256), 256, 0, h->n, h->keyU, h->idU, h->crange, h->hist, h->tmp, h->tmpid, h->err);
 }
 
+sph::WallLists wall_lists(const SphHandle* h) { return {h->wcount, h->nb ? h->wlist : nullptr}; }
+
 void enqueue_density_only(SphHandle* h) {
   using namespace sph;
   int bs = h->bs_density;
   sph::ClosureBufs cb{h->cl_count, h->cl_slot, h->cl_feat, h->cl_rho, h->corr, h->vel, h->cl_wq, h->cl_wf};
+  const WallLists wl = wall_lists(h);
   if (h->cl_mode) cudaMemsetAsync(h->cl_count, 0, sizeof(uint32_t), h->st);
   // the warp scan's scratch per warp; closure mode 2 adds a 16-sample network
   // tile per warp (the fused inference)
@@ -696,7 +699,7 @@ void enqueue_density_only(SphHandle* h) {
         auto run = [&](auto kernel, size_t smem) {
           launch(h, kernel, grid, kGroupThreads, smem, kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
                  h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
-                 h->slow);
+                 h->slow, wl);
         };
         if (h->cl_mode == 2) run(k_density_group<KPT, 2, G>, smem1 + sizeof(BlockTile));
         else if (h->cl_mode) run(k_density_group<KPT, 1, G>, smem1);
@@ -712,7 +715,7 @@ void enqueue_density_only(SphHandle* h) {
       auto run = [&](auto kernel, size_t smem) {
         launch(h, kernel, grid_for(h->n, kGroupThreads / 32 * kPairParticles), kGroupThreads, smem, kp, h->n, h->dt,
                h->pos, planes(h), h->rv, h->id, h->ctab, h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err,
-               h->nbr, h->ncount, h->sdf, h->wall_tab, cb, h->slow);
+               h->nbr, h->ncount, h->sdf, h->wall_tab, cb, h->slow, wl);
       };
       if (h->cl_mode == 2) run(k_density_pair<KPT, 2>, bytes + (kGroupThreads / 32) * kClTileWords * sizeof(uint32_t));
       else if (h->cl_mode) run(k_density_pair<KPT, 1>, bytes);
@@ -738,11 +741,11 @@ void enqueue_density_only(SphHandle* h) {
 void enqueue_adami(SphHandle* h) {
   using namespace sph;
   if (h->nb == 0) return;
-  if (h->wlist) {
+  if (h->wlist && (h->lanes_density == 1 || h->cl_mode)) {  // else the density pass has done it (scatter_walls)
     const int P = h->n >= 1000000 ? 16 : 8;  // between 250k and 2M particles the two cross (k_wall_scatter)
     dispatch(h, false, [&](auto kp) {
       launch(h, k_wall_scatter<decltype(kp)>, grid_for(h->n, 8 * P), 256, 0, kp, h->n, P, h->pos, h->nbr, h->ncount,
-             h->bc_start, h->bc_list, h->bpos, h->wcount, h->wlist, h->err);
+             h->bc_start, h->bc_list, h->bpos, wall_lists(h), h->err);
     });
   }
   dispatch(h, true, [&](auto kp) {

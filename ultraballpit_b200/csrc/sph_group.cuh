@@ -265,7 +265,7 @@ k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __res
                 const float4* __restrict__ bpos, float2* __restrict__ rf, float* __restrict__ pr,
                 const uint32_t* __restrict__ err, uint32_t* __restrict__ nbr, uint32_t* __restrict__ ncount,
                 const float* __restrict__ sdf, const float2* __restrict__ wall_tab, ClosureBufs cb,
-                uint32_t* __restrict__ slow) {
+                uint32_t* __restrict__ slow, WallLists wl) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int NC = CL ? 3 : 2, P = 32 / G;
   extern __shared__ __align__(16) unsigned char s_dyn[];
@@ -464,6 +464,12 @@ k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __res
         reinterpret_cast<uint4*>(nbr)[(size_t)q * (size_t)n + (size_t)ip] =
             *reinterpret_cast<const uint4*>(&S.list[p][q * 4]);
   }
+  const uint32_t counts = live ? pack_counts(listed, nwall, close) : 0u;
+  if (CL == 0 && wl.list) {
+    const uint32_t theirs = __shfl_sync(kAll, counts, (lane % P) * G);
+    scatter_walls(kp, base, lane < P ? theirs : 0u, pos, bc_start, bc_list, bpos, wl,
+                  [&](int src, uint32_t e) { return S.list[src][e]; });
+  }
   rho = g.get(wsum, 0);
   const DensityState st{rho, diff_sum, ssum, CL ? g.get(wsum, 1) : 0.0f, nwall, listed};
   const float centre = live ? centre_sdf<CL>(k, sdf, pi) : 0.0f;
@@ -475,7 +481,7 @@ k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __res
   float rho_pre = 0.0f;
   bool near_wall = false;
   if (live && g.sub == 0) {
-    ncount[i] = pack_counts(listed, nwall, close);
+    ncount[i] = counts;
     near_wall = density_finish<CL>(k, i, dtp[k.inst], pi, st, rv, id, rf, pr, centre,
                                    [&](int a) { return probes[CL ? a : 0]; }, wall_tab, cb, slow, f, rho_pre);
   }
@@ -526,7 +532,7 @@ k_density_pair(KP kp, int n, const float* __restrict__ dtp, const float4* __rest
                const float4* __restrict__ bpos, float2* __restrict__ rf, float* __restrict__ pr,
                const uint32_t* __restrict__ err, uint32_t* __restrict__ nbr, uint32_t* __restrict__ ncount,
                const float* __restrict__ sdf, const float2* __restrict__ wall_tab, ClosureBufs cb,
-               uint32_t* __restrict__ slow) {
+               uint32_t* __restrict__ slow, WallLists wl) {
   constexpr unsigned kAll = 0xffffffffu;
   constexpr int P = kPairParticles;
   extern __shared__ __align__(16) unsigned char s_dyn[];
@@ -721,6 +727,12 @@ k_density_pair(KP kp, int n, const float* __restrict__ dtp, const float4* __rest
     if (inb && e < kNbrCap) nbr[nbr_index(e, n, i)] = ib;
     nwall += first + ((ma >> (p + P)) & 1u) + ((mb >> (p + P)) & 1u);
   }
+  const uint32_t counts = live && !second ? pack_counts(listed, nwall, close) : 0u;
+  if (CL == 0 && wl.list) {
+    __syncwarp();
+    scatter_walls(kp, base, counts, pos, bc_start, bc_list, bpos, wl,
+                  [&](int src, uint32_t e) { return nbr[nbr_index(e, n, base + src)]; });
+  }
   const float centre = live ? centre_sdf<CL>(k, sdf, pi) : 0.0f;
   float probes[CL ? 12 : 1];
   if (CL)
@@ -730,7 +742,7 @@ k_density_pair(KP kp, int n, const float* __restrict__ dtp, const float4* __rest
   float rho_pre = 0.0f;
   bool near_wall = false;
   if (live && !second) {
-    ncount[i] = pack_counts(listed, nwall, close);
+    ncount[i] = counts;
     near_wall = density_finish<CL>(k, i, dtp[k.inst], pi, DensityState{rho, diff_sum, ssum, rho_wall, nwall, listed},
                                    rv, id, rf, pr, centre, [&](int a) { return probes[CL ? a : 0]; }, wall_tab, cb,
                                    slow, f, rho_pre);
