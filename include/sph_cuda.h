@@ -204,7 +204,9 @@ int sph_create(const SphParams *params, const SphParticlesView *particles,
 /* Releases the handle. Its device arrays go back to the library's pool,
  * which keeps them for the next handle created on that device (creating
  * simulations one after another then skips the driver's mapping of fresh
- * memory); the pool's memory stays reserved until the process exits. */
+ * memory); the pool's memory stays reserved until the process exits. The
+ * page-locked staging of reads to the host goes with the last handle that
+ * counts on it. */
 void sph_destroy(SphHandle *h);
 
 /* SimulationKernel::step (lib.rs:287-335). Enqueued asynchronously. */
@@ -328,7 +330,8 @@ int sph_batch_info(const SphHandle *h, int *ninst, size_t *first, size_t *count)
 int sph_batch_step(SphHandle *h, const float *dts);
 /* Per-instance sph::compute_timestep on the device (ninst floats). */
 int sph_batch_timesteps(SphHandle *h, float *dt_out);
-/* Launch shapes of the neighbour kernels (graphs are recaptured). */
+/* Launch shapes of the neighbour kernels with one lane per particle (graphs
+ * are recaptured); those with several have a fixed shape. */
 int sph_set_launch(SphHandle *h, const SphLaunch *launch);
 int sph_get_launch(const SphHandle *h, SphLaunch *launch);
 /* Autotuner: times each kernel at 64/128/256/512 threads per block over

@@ -1,8 +1,8 @@
 // sph_api.cu - host side of libsph_cuda.so: the C ABI of include/sph_cuda.h.
 //
 // One SphHandle = one simulation on one device: its own stream, device
-// buffers and CUDA graphs. The step body (9 kernels) is captured once into a
-// graph and replayed; dt lives in device memory so the graph never changes.
+// buffers and CUDA graphs. The step body (7 to 11 kernels by size) is captured
+// once into a graph and replayed; dt lives in device memory so the graph never changes.
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -84,7 +84,7 @@ struct SphHandle {
   uint32_t *rank_of_lin = nullptr, *lin_of_rank = nullptr;
   uint2* ctab = nullptr;
   int nbsum = 0;
-  // neighbour lists recorded by k_density (entry-major, sph::nbr_index), count per particle
+  // neighbour lists recorded by k_density (quad-major, sph::nbr_index), count per particle
   uint32_t *nbr = nullptr, *ncount = nullptr;
   // XSPH gather records: (x, y, z, m), (v + a dt/2, rho) per particle
   float4* xrec = nullptr;
@@ -634,30 +634,34 @@ void choose_lanes(SphHandle* h, int sms) {
   }
 }
 
-// Lets the density kernels take up to 128 KiB of dynamic shared memory (the
-// warp scan's per-warp scratch passes the default 48 KiB at 512 threads) on
-// the current device. Set at handle creation, before any graph capture.
-void allow_density_smem() {
+// Lets the handle's density kernels take up to 128 KiB of dynamic shared memory
+// (the warp scan's per-warp scratch passes the default 48 KiB at 512 threads)
+// on the current device. Set at handle creation, before any graph capture, and
+// only for the form in use: naming a kernel here loads it (all 18: a process's
+// first creation 34 ms, these three: 31).
+void allow_density_smem(const SphHandle* h) {
   using namespace sph;
-  auto set = [](const void* f) {
-    cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+  auto set = [](auto kernel) {
+    cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         128 * 1024);
   };
-  set(reinterpret_cast<const void*>(k_density<OneSim, 0>));
-  set(reinterpret_cast<const void*>(k_density<OneSim, 1>));
-  set(reinterpret_cast<const void*>(k_density<OneSim, 2>));
-  set(reinterpret_cast<const void*>(k_density<ManySim, 0>));
-  set(reinterpret_cast<const void*>(k_density<ManySim, 1>));
-  set(reinterpret_cast<const void*>(k_density<ManySim, 2>));
-  auto group = [&](auto lanes) {
-    constexpr int G = decltype(lanes)::value;
-    set(reinterpret_cast<const void*>(k_density_group<OneSim, 0, G>));
-    set(reinterpret_cast<const void*>(k_density_group<OneSim, 1, G>));
-    set(reinterpret_cast<const void*>(k_density_group<OneSim, 2, G>));
-    set(reinterpret_cast<const void*>(k_density_group<ManySim, 0, G>));
-    set(reinterpret_cast<const void*>(k_density_group<ManySim, 1, G>));
-    set(reinterpret_cast<const void*>(k_density_group<ManySim, 2, G>));
+  auto form = [&](auto* constants) {
+    using KPT = std::remove_pointer_t<decltype(constants)>;
+    if (h->lanes_density > 2) {
+      with_lanes(h->lanes_density, [&](auto lanes) {
+        constexpr int G = decltype(lanes)::value;
+        set(k_density_group<KPT, 0, G>);
+        set(k_density_group<KPT, 1, G>);
+        set(k_density_group<KPT, 2, G>);
+      });
+    } else if (h->lanes_density == 1) {
+      set(k_density<KPT, 0>);
+      set(k_density<KPT, 1>);
+      set(k_density<KPT, 2>);
+    }
   };
-  for (int lanes : {8, 16}) with_lanes(lanes, group);
+  if (h->ninst == 1) form(static_cast<OneSim*>(nullptr));
+  else form(static_cast<ManySim*>(nullptr));
 }
 
 // Sorting scratch + binning of posU into the cell tables (k_bin or the
@@ -1190,10 +1194,10 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
       return;
     }
     ae = cudaStreamCreateWithFlags(&h->st, cudaStreamNonBlocking);
-    allow_density_smem();
     int sms = 148;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess) sms = 148;
     choose_lanes(h, sms);
+    allow_density_smem(h);
 #define ALLOC(ptr, cnt) \
   if (ae == cudaSuccess) ae = dalloc(h, &h->ptr, (cnt))
     ALLOC(pos, n); ALLOC(vel, n); ALLOC(velout, n); ALLOC(acc, n);
