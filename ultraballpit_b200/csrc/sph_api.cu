@@ -802,9 +802,9 @@ void enqueue_xsph(SphHandle* h, bool use_list, bool auto_dt = false) {
     dispatch(h, false, [&](auto kp) {
       with_lanes(h->lanes_xsph, [&](auto lanes) {
         constexpr int G = decltype(lanes)::value;
-        launch(h, k_xsph_group<decltype(kp), G>, grid_for(h->n, kGroupThreads / G), kGroupThreads, 0, kp, h->n, h->dt,
-               auto_dt ? h->red : nullptr, h->pos, h->velout, h->acc, h->id, h->ctab, h->rank_of_lin, h->posU,
-               h->velU, h->idU, h->keyU, h->hist, h->err, h->nbr, h->ncount);
+        launch(h, k_xsph_group<decltype(kp), G>, grid_for(h->n, kGroupThreads / G), kGroupThreads, 0, kp, h->n,
+               h->ninst, h->dt, auto_dt ? h->red : nullptr, h->pos, h->velout, h->acc, h->id, h->ctab, h->rank_of_lin,
+               h->posU, h->velU, h->idU, h->keyU, h->hist, h->err, h->nbr, h->ncount);
       });
     });
     return;

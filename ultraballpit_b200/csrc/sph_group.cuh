@@ -116,10 +116,12 @@ __device__ __forceinline__ void group_candidates(const Group<G>& g, uint32_t q0,
 // The neighbours' half-kicked velocities (k_xsph_prep's records in the thread
 // form) are computed here from velocity and acceleration: a launch less, where
 // launches count. With `red` the kernel also computes the step's dt from the
-// last step's maxima, for every instance's own particles, and stores it.
+// last step's maxima, for every instance's own particles; the first block
+// stores it, for all `ninst` instances, those without particles among them.
 template <class KP, int G>
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
-k_xsph_group(KP kp, int n, float* __restrict__ dtp, const float* __restrict__ red, const float4* __restrict__ pos,
+k_xsph_group(KP kp, int n, int ninst, float* __restrict__ dtp, const float* __restrict__ red,
+             const float4* __restrict__ pos,
              const float4* __restrict__ velout, const float4* __restrict__ acc,
              const uint32_t* __restrict__ id, const uint2* __restrict__ ctab,
              const uint32_t* __restrict__ rank_of_lin, float4* __restrict__ posU, float4* __restrict__ velU,
@@ -137,7 +139,9 @@ k_xsph_group(KP kp, int n, float* __restrict__ dtp, const float* __restrict__ re
   float dt;
   if (red) {
     dt = cfl_dt(k.h, k.c, k.cfl, red[2 * k.inst], red[2 * k.inst + 1]);
-    if (live && g.sub == 0 && kp.first(i)) dtp[k.inst] = dt;
+    if (blockIdx.x == 0)
+      for (int q = threadIdx.x; q < ninst; q += kGroupThreads)
+        dtp[q] = cfl_dt(kp.tab[q].h, kp.tab[q].c, kp.tab[q].cfl, red[2 * q], red[2 * q + 1]);
   } else {
     dt = dtp[k.inst];
   }
