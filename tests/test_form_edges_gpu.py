@@ -5,10 +5,12 @@ ordinary, and the paths taken only by large grids or without a boundary list."""
 import numpy as np
 import pytest
 
-from ultraballpit_b200.kernel import CudaBatch
+from oracle import oracle as orc
+from ultraballpit_b200.kernel import CudaBatch, CudaKernel
+from ultraballpit_b200.particles import BoundaryParticles, ParticleArrays
 
 from test_group_forms_gpu import first
-from test_parity_gpu import small_dam_break
+from test_parity_gpu import assert_same, small_dam_break
 
 pytestmark = pytest.mark.gpu
 
@@ -28,3 +30,29 @@ def test_timestep_of_an_instance_without_particles(lanes, empty, monkeypatch):
     dt = b.step_auto(1)
     assert f(dt) == want[0]
     b.close()
+
+
+@pytest.mark.parametrize("lanes", ["1", "2", "8", "16"])
+def test_close_pair_in_a_crowded_neighbourhood(lanes, monkeypatch):
+    """Three particles 1e-13 and 3e-12 apart, alone in their support, with 900 more beyond it in the cells around:
+    too many candidates for the scan's masks, and a distance below 1e-12, where the kernel's gradient is zero."""
+    monkeypatch.setenv("SPH_GROUP_LANES", lanes)
+    h = np.float32(1.3 * 0.004)
+    cell = np.float32(2.0) * h
+    rng = np.random.default_rng(1)
+    x, y, z = (rng.uniform(lo, 0.0205, 903).astype(np.float32) for lo in (0.015, 0.0, 0.0))
+    x[:3], y[:3], z[:3] = (0.0, 1e-13, 0.0), (0.0, 0.0, 3e-12), 0.0
+    p = ParticleArrays.from_positions(x, y, z, 6.4e-5)
+    p.mass[:3] *= 4  # their density above the rest density, so that they press on one another
+    p.mass[3:] *= np.float32(0.05)
+    p.vx[0], p.vy[2] = 0.5, -0.5
+    none = BoundaryParticles.from_arrays(*[np.zeros(0, np.float32)] * 7)
+    args = (p, none, float(h), (0.0, 0.0, -9.81), 20.0, 0.25, 0.0, (float(-2 * cell),) * 3, (float(8 * cell),) * 3)
+    gpu = CudaKernel(*args)
+    cpu = orc.OracleKernel(*args, tier=1, threads=8, pow_mode=1)
+    assert [len(gpu.neighbors(q)) for q in range(3)] == [2, 2, 2]
+    for _ in range(3):
+        gpu.step(1e-7)
+        cpu.step(1e-7)
+        assert_same(gpu.particles(), cpu.particles())
+    gpu.close()

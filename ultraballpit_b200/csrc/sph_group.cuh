@@ -596,7 +596,14 @@ k_density_pair(KP kp, int n, const float* __restrict__ dtp, const float4* __rest
     const bool act = in_batch && nw <= kScanWords;
     if (in_batch && !act) {
       fed = false;
-      if (!second) dense = record_neighbors(pi.x, pi.y, pi.z, i, pl, ctab, ScanGeo(k), nbr, n);
+      if (!second) {
+        dense = record_neighbors(pi.x, pi.y, pi.z, i, pl, ctab, ScanGeo(k), nbr, n);
+        for (uint32_t e = 0; e < min(dense, kNbrCap); ++e) {  // no terms here: the closest is looked for by itself
+          const float4 pj = __ldg(&pos[nbr[nbr_index(e, n, i)]]);
+          const float dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+          dmin = fminf(dmin, dx * dx + dy * dy + dz * dz);
+        }
+      }
     }
     __syncwarp();
     const uint32_t q4 = act ? S.mquad[s] : 0u;
