@@ -9,6 +9,7 @@
 #include <cmath>
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include <cuda_bf16.h>
@@ -33,7 +34,8 @@ struct SphMlp {
   size_t loss_tiles = 0;
   // samples, targets (or outputs) and permutation on the device; these, the
   // partials and the losses are pieces of `work`, kept from call to call up to
-  // kKeep bytes
+  // kKeep bytes. `mu` is held by the call that uses them.
+  std::mutex mu;
   unsigned char* work = nullptr;
   size_t work_bytes = 0;
   float *dx = nullptr, *dt = nullptr;
@@ -547,21 +549,34 @@ int sph_mlp_forward(SphMlp* h, const float* x, size_t n, float* y) {
   if (!h || (n && (!x || !y)) || n > 0x7fffffffull) return SPH_ERR_INVALID_ARG;
   if (n == 0) return SPH_OK;
   cudaSetDevice(h->dev);
+  auto run = [&](float* dx, float* dy) {
+    cudaError_t e = cudaMemcpyAsync(dx, x, n * kIn * sizeof(float), cudaMemcpyHostToDevice, h->st);
+    if (e == cudaSuccess) {
+      int blocks = (int)std::min<size_t>((n + kCtaSamples - 1) / kCtaSamples, (size_t)h->sms * 4);
+      k_mlp_forward<<<blocks, kWarps * 32, sizeof(CtaSmem), h->st>>>(h->wb, h->w, dx, (int)n, dy);
+      e = cudaMemcpyAsync(y, dy, n * kOut * sizeof(float), cudaMemcpyDeviceToHost, h->st);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+    return e;
+  };
+  std::unique_lock<std::mutex> lock(h->mu, std::try_to_lock);
+  if (!lock.owns_lock()) {  // another thread's call has the kept buffers, perhaps for a whole training
+    float* own = nullptr;
+    cudaError_t e = cudaMalloc((void**)&own, n * (kIn + kOut) * sizeof(float));
+    if (e == cudaSuccess) e = run(own, own + n * kIn);
+    if (own) cudaFree(own);
+    return status(e);
+  }
   KeepSmall keep{h};
   cudaError_t e = ensure_work(h, n, 0, 0);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(h->dx, x, n * kIn * sizeof(float), cudaMemcpyHostToDevice, h->st);
-  if (e == cudaSuccess) {
-    int blocks = (int)std::min<size_t>((n + kCtaSamples - 1) / kCtaSamples, (size_t)h->sms * 4);
-    k_mlp_forward<<<blocks, kWarps * 32, sizeof(CtaSmem), h->st>>>(h->wb, h->w, h->dx, (int)n, h->dt);
-    e = cudaMemcpyAsync(y, h->dt, n * kOut * sizeof(float), cudaMemcpyDeviceToHost, h->st);
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
+  if (e == cudaSuccess) e = run(h->dx, h->dt);
   return status(e);
 }
 
 int sph_mlp_loss_grad(SphMlp* h, const float* x, const float* t, size_t n, float* loss, float* grad) {
   if (!h || !x || !t || n == 0 || n > (1u << 24)) return SPH_ERR_INVALID_ARG;
   cudaSetDevice(h->dev);
+  std::lock_guard<std::mutex> lock(h->mu);
   KeepSmall keep{h};
   const size_t tiles = (n + 15) / 16;
   cudaError_t e = ensure_work(h, n, Split(h, n).rows, tiles);
@@ -588,6 +603,7 @@ int sph_mlp_train(SphMlp* h, const float* x, const float* t, size_t n, int batch
   if (!h || !x || !t || n == 0 || n > 0x7fffffffull || batch < 16 || epochs < 1 || !(lr > 0.0f))
     return SPH_ERR_INVALID_ARG;
   cudaSetDevice(h->dev);
+  std::lock_guard<std::mutex> lock(h->mu);
   KeepSmall keep{h};
   // tiles of an epoch, mini-batch by mini-batch
   const size_t full = n / (size_t)batch, per = ((size_t)batch + 15) / 16, rest = n % (size_t)batch;
