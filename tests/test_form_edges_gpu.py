@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 
 from oracle import oracle as orc
+from ultraballpit_b200 import domain
 from ultraballpit_b200.kernel import CudaBatch, CudaKernel
 from ultraballpit_b200.particles import BoundaryParticles, ParticleArrays
 
@@ -56,3 +57,49 @@ def test_close_pair_in_a_crowded_neighbourhood(lanes, monkeypatch):
         cpu.step(1e-7)
         assert_same(gpu.particles(), cpu.particles())
     gpu.close()
+
+
+def forces_us(k):
+    return min(k.step_profiled(2e-5)["forces_us"] for _ in range(12))
+
+
+def alone(sc, q, mass):
+    """Particles q of the scenario in the middle of its empty part, with the given mass."""
+    p = sc.particles
+    p.mass[q], p.x[q], p.y[q], p.z[q] = mass, 0.25, 0.1, 0.05
+
+
+def passing(sc):  # two particles in one place, denser together than 2^30, that part at once
+    alone(sc, [4, 5], 200.0)
+    sc.particles.vx[4], sc.particles.vx[5] = -700.0, 700.0
+
+
+def thin(sc):  # a particle by itself whose density is far below any fluid's
+    alone(sc, [4], 1e-15)
+
+
+def light(sc):  # masses of a very fine discretisation
+    alone(sc, [4], 1e-20)
+
+
+@pytest.mark.parametrize("lanes", ["1", "8"])
+@pytest.mark.parametrize("change", [passing, thin, light])
+def test_an_odd_particle_does_not_slow_the_rest(change, lanes, monkeypatch):
+    """The sums of all particles leave their lists for a grid search (5 to 9 times the forces' time) while a density
+    or mass of the simulation is outside what the quick quotients allow, and only then."""
+    monkeypatch.setenv("SPH_GROUP_LANES", lanes)
+    times = []
+    for f in (None, change):
+        sc = domain.dam_break(0.004, seed=3, block=(0.1, 0.2, 0.1), domain_max=(0.4, 0.2, 0.1), with_sdf=False)
+        if f:
+            f(sc)
+        gpu = CudaKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta)
+        if f:
+            cpu = orc.OracleKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta, tier=1, threads=8, pow_mode=1)
+            for _ in range(3):
+                gpu.step(2e-5)
+                cpu.step(2e-5)
+                assert_same(gpu.particles(), cpu.particles())
+        times.append(forces_us(gpu))
+        gpu.close()
+    assert times[1] < 2.0 * times[0], times

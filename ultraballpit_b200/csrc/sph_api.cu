@@ -132,7 +132,9 @@ struct SphHandle {
   float* var = nullptr;
   uint32_t* err = nullptr;
   float *dt = nullptr, *dt_query = nullptr, *red = nullptr;
-  uint32_t* slow = nullptr;  // per instance: its pair sums take the general operations (k_xsph_prep, k_density)
+  // per instance: its pair sums take the general operations (set by k_xsph_prep
+  // and the density pass, taken back by k_reorder)
+  uint32_t* slow = nullptr;
   // metrics
   int nparts = 0;
   double *part_m = nullptr, *part_e = nullptr;
@@ -821,12 +823,13 @@ void enqueue_xsph(SphHandle* h, bool use_list, bool auto_dt = false) {
   });
 }
 
-// The sort; it also clears `red` for enqueue_forces.
+// The sort; it also clears `red` for enqueue_forces and takes back `slow`.
 void enqueue_sort(SphHandle* h) {
   using namespace sph;
   enqueue_scan_fill(h);
   launch(h, k_reorder, grid_for(h->n, 256), 256, 0, h->n, h->tmp, h->tmpid, h->crange, h->posU, h->velU, h->pos,
-         h->vel, h->rv, h->id, h->err, nullptr, nullptr, nullptr, nullptr, nullptr, planes(h), h->red, 2 * h->ninst);
+         h->vel, h->rv, h->id, h->err, nullptr, nullptr, nullptr, nullptr, nullptr, planes(h), h->red, h->slow, h->ktab,
+         h->ninst);
 }
 
 // lib.rs:287-335 after the bootstrap: kick1+XSPH+drift+clamp, grid + reorder,
@@ -1478,7 +1481,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     h->launches += 1;
     enqueue_scan_fill(h);
     launch(h, k_reorder, grid_for(h->n, 256), 256, 0, h->n, h->tmp, h->tmpid, h->crange, h->posU, h->velU, h->pos,
-           h->vel, h->rv, h->id, h->err, accU, h->acc, prU, h->pr, h->velout, planes(h), nullptr, 0);
+           h->vel, h->rv, h->id, h->err, accU, h->acc, prU, h->pr, h->velout, planes(h), nullptr, nullptr, nullptr, 0);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
