@@ -103,3 +103,33 @@ def test_an_odd_particle_does_not_slow_the_rest(change, lanes, monkeypatch):
         times.append(forces_us(gpu))
         gpu.close()
     assert times[1] < 2.0 * times[0], times
+
+
+@pytest.mark.parametrize("lanes", ["1", "8"])
+@pytest.mark.parametrize("coef", [(-0.5, 2.0), (0.5, -2.0), (-0.5, -2.0), (-1e-25, 1.0), (1e-25, -1.0)])
+def test_negative_viscous_coefficients(coef, lanes, monkeypatch):
+    """Velocities over 34 decades: viscous dividends whose two parts cancel or underflow, some to nothing."""
+    monkeypatch.setenv("SPH_GROUP_LANES", lanes)
+    sc = small_dam_break()
+    p, rng = sc.particles, np.random.default_rng(9)
+    for a in (p.vx, p.vy, p.vz):
+        a[:] = (rng.uniform(-1, 1, len(p)) * 10.0 ** rng.uniform(-34, 0, len(p))).astype(np.float32)
+    gpu = CudaKernel(*sc.kernel_args(), alpha=coef[0], beta=coef[1])
+    cpu = orc.OracleKernel(*sc.kernel_args(), alpha=coef[0], beta=coef[1], tier=1, threads=8, pow_mode=1)
+    for _ in range(3):
+        gpu.step(2e-5)
+        cpu.step(2e-5)
+        assert_same(gpu.particles(), cpu.particles())
+    gpu.close()
+
+
+@pytest.mark.parametrize("lanes", ["1", "8"])
+def test_negative_viscous_coefficients_keep_the_lists(lanes, monkeypatch):
+    monkeypatch.setenv("SPH_GROUP_LANES", lanes)
+    times = []
+    for alpha in (0.5, -0.5):
+        sc = domain.dam_break(0.004, seed=3, block=(0.1, 0.2, 0.1), domain_max=(0.4, 0.2, 0.1), with_sdf=False)
+        gpu = CudaKernel(*sc.kernel_args(), alpha=alpha, beta=sc.beta)
+        times.append(forces_us(gpu))
+        gpu.close()
+    assert times[1] < 2.0 * times[0], times

@@ -290,15 +290,19 @@ SimConst make_const(const SphParams& p, const uint32_t dims[3]) {
   // most b, so a dividend of 2^-98 max(b, 1) has a normal quotient and exact
   // residuals, and a viscous dividend of mu_min b a |mu| of at least mu_min,
   // from which on the second dividend alpha c |mu| + beta mu^2 is at least
-  // 2^-94 (a normal quotient by any density sum up to 2 kRhoMax). Negative or
-  // non-finite coefficients could cancel: those take the general operations.
+  // 2^-94 (a normal quotient by any density sum up to 2 kRhoMax). With a
+  // negative coefficient the two may cancel: forces_fast then watches their
+  // sum. Non-finite or huge ones take the general operations.
   k.neg_alpha_c2 = 2.0f * k.neg_alpha_c;
   k.beta2 = 2.0f * k.beta;
   const double ac = -(double)k.neg_alpha_c, be = (double)k.beta, b = 4.1 * (double)h * h;
-  k.fast = h >= 0x1p-24f && h <= 0x1p20f && ac >= 0.0 && ac <= 0x1p60 && be >= 0.0 && be <= 0x1p60;
+  k.fast = h >= 0x1p-24f && h <= 0x1p20f && std::fabs(ac) <= 0x1p60 && std::fabs(be) <= 0x1p60;
+  k.mixed = ac < 0.0 || be < 0.0;
   double mu_min = 0.0;
-  if (ac > 0.0) mu_min = 0x1p-94 / ac;
-  if (be > 0.0) mu_min = ac > 0.0 ? std::min(mu_min, std::sqrt(0x1p-94 / be)) : std::sqrt(0x1p-94 / be);
+  if (!k.mixed) {
+    if (ac > 0.0) mu_min = 0x1p-94 / ac;
+    if (be > 0.0) mu_min = ac > 0.0 ? std::min(mu_min, std::sqrt(0x1p-94 / be)) : std::sqrt(0x1p-94 / be);
+  }
   auto key_of = [](double v) {
     const float f = (float)std::min(1e30, v);
     uint32_t bits;
@@ -768,6 +772,7 @@ void enqueue_density_adami(SphHandle* h) {
 // `red` is clear when it runs (clear_red, or k_reorder).
 void enqueue_forces(SphHandle* h, float hdt_scale) {
   using namespace sph;
+  const bool mixed = std::any_of(h->ktab_h.begin(), h->ktab_h.end(), [](const SimConst& k) { return k.mixed != 0; });
   dispatch(h, false, [&](auto kp) {
     using KPT = decltype(kp);
     auto run = [&](auto kernel, int grid, int block) {
@@ -779,13 +784,13 @@ void enqueue_forces(SphHandle* h, float hdt_scale) {
       with_lanes(h->lanes_forces, [&](auto lanes) {
         constexpr int G = decltype(lanes)::value;
         const int grid = grid_for(h->n, kGroupThreads / G);
-        if (h->cl_mode) run(k_forces_group<KPT, 1, G>, grid, kGroupThreads);
-        else run(k_forces_group<KPT, 0, G>, grid, kGroupThreads);
+        if (h->cl_mode) run(mixed ? k_forces_group<KPT, 1, G, true> : k_forces_group<KPT, 1, G, false>, grid, kGroupThreads);
+        else run(mixed ? k_forces_group<KPT, 0, G, true> : k_forces_group<KPT, 0, G, false>, grid, kGroupThreads);
       });
     } else {
       const int bs = h->bs_forces;
-      if (h->cl_mode) run(k_forces<KPT, 1>, grid_for(h->n, bs), bs);
-      else run(k_forces<KPT, 0>, grid_for(h->n, bs), bs);
+      if (h->cl_mode) run(mixed ? k_forces<KPT, 1, true> : k_forces<KPT, 1, false>, grid_for(h->n, bs), bs);
+      else run(mixed ? k_forces<KPT, 0, true> : k_forces<KPT, 0, false>, grid_for(h->n, bs), bs);
     }
   });
 }

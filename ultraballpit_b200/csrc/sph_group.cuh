@@ -773,7 +773,7 @@ struct __align__(16) ForceGroup {
   uint32_t rep[kRepCap];  // boundary candidates within the repulsion radius, in order
 };
 
-template <class KP, int CL, int G>
+template <class KP, int CL, int G, bool MIXED>
 __global__ void __launch_bounds__(kGroupThreads, kGroupBlocks)
 k_forces_group(KP kp, int n, const float* __restrict__ dtp, float hdt_scale, const float4* __restrict__ pos,
                const float4* __restrict__ vel, const float2* __restrict__ rf, const float* __restrict__ pr,
@@ -825,8 +825,8 @@ k_forces_group(KP kp, int n, const float* __restrict__ dtp, float hdt_scale, con
       const float dx = pi.x - pj[u].x, dy = pi.y - pj[u].y, dz = pi.z - pj[u].z;
       uint32_t kk = 0xffffffffu;
       float factor, fv, gx, gy, gz;
-      forces_fast(k, neg_mi, vi, rfi, pj[u], vj[u], rfj[u], dx, dy, dz, dx * dx + dy * dy + dz * dz, kk, factor, fv,
-                  gx, gy, gz);
+      forces_fast<MIXED>(k, neg_mi, vi, rfi, pj[u], vj[u], rfj[u], dx, dy, dz, dx * dx + dy * dy + dz * dz, kk, factor,
+                         fv, gx, gy, gz);
       if (in) key = min(key, kk);
       S.terms.t[0][u * G + g.sub] = in ? factor * gx : 0.0f;
       S.terms.t[1][u * G + g.sub] = in ? factor * gy : 0.0f;
