@@ -336,7 +336,8 @@ int sph_set_launch(SphHandle *h, const SphLaunch *launch);
 int sph_get_launch(const SphHandle *h, SphLaunch *launch);
 /* Autotuner: times each kernel at 64/128/256/512 threads per block over
  * `trial_steps` profiled steps (after one untimed step) and applies the
- * fastest shape per kernel. Results are cached per process by device name
+ * fastest shape per kernel; a kernel with several lanes per particle keeps
+ * its own. Results are cached per process by device name, lanes per particle
  * and instance-size histogram; a cache hit runs no step. The trial steps
  * advance the simulation: tune a scratch handle of the same workload. */
 int sph_autotune(SphHandle *h, int trial_steps, SphLaunch *best);

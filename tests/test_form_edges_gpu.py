@@ -133,3 +133,20 @@ def test_negative_viscous_coefficients_keep_the_lists(lanes, monkeypatch):
         times.append(forces_us(gpu))
         gpu.close()
     assert times[1] < 2.0 * times[0], times
+
+
+def test_tuned_shapes_belong_to_the_form(monkeypatch):
+    """The forms change inside a bin of the size histogram: shapes tuned for one are not handed to another."""
+    sc = first(small_dam_break(), 777)
+    best = {}
+    for lanes in ("8", "1", "8", "1"):
+        monkeypatch.setenv("SPH_GROUP_LANES", lanes)
+        k = CudaKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta)
+        before = k.particles()
+        got = k.autotune(2)
+        k._cache = None
+        cached = np.array_equal(before.z, k.particles().z)
+        assert cached == (lanes in best)  # a cache hit runs no step
+        assert best.setdefault(lanes, got) == got == k.launch()
+        assert lanes == "1" or set(got.values()) == {128}  # nothing to choose
+        k.close()

@@ -2229,8 +2229,9 @@ int sph_get_launch(const SphHandle* h, SphLaunch* l) {
   return SPH_OK;
 }
 
-// Autotuner cache: (device name, instance count, log2 histogram of instance
-// sizes) -> best launch shapes.
+// Autotuner cache: (device name, instance count, lanes per particle of the three
+// kernels, log2 histogram of instance sizes) -> best launch shapes. The lanes
+// change inside a bin of the histogram, and a kernel with several has one shape.
 static std::mutex g_tune_mu;
 static std::map<std::string, SphLaunch> g_tune_cache;
 
@@ -2245,6 +2246,7 @@ static std::string tune_key(SphHandle* h) {
     hist[b]++;
   }
   key += "|" + std::to_string(h->ninst);
+  for (int lanes : {h->lanes_xsph, h->lanes_density, h->lanes_forces}) key += "/" + std::to_string(lanes);
   for (int b = 0; b < 40; ++b)
     if (hist[b]) key += "|" + std::to_string(b) + ":" + std::to_string(hist[b]);
   return key;
@@ -2286,9 +2288,11 @@ int sph_autotune(SphHandle* h, int trial_steps, SphLaunch* best) {
     for (int a = 0; a < 3; ++a)
       if (acc[a] < t_best[a]) { t_best[a] = acc[a]; s_best[a] = c; }
   }
-  best->xsph_threads = s_best[0];
-  best->density_threads = s_best[1];
-  best->forces_threads = s_best[2];
+  // a kernel with several lanes per particle ran the same launch every time
+  const SphHandle d;
+  best->xsph_threads = h->lanes_xsph > 1 ? d.bs_xsph : s_best[0];
+  best->density_threads = h->lanes_density > 1 ? d.bs_density : s_best[1];
+  best->forces_threads = h->lanes_forces > 1 ? d.bs_forces : s_best[2];
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_tune_cache[key] = *best;
