@@ -7,6 +7,7 @@ import pytest
 
 from oracle import oracle as orc
 from ultraballpit_b200 import domain
+from ultraballpit_b200.closure import ClosureNet
 from ultraballpit_b200.kernel import CudaBatch, CudaKernel
 from ultraballpit_b200.particles import BoundaryParticles, ParticleArrays
 
@@ -150,3 +151,22 @@ def test_tuned_shapes_belong_to_the_form(monkeypatch):
         assert best.setdefault(lanes, got) == got == k.launch()
         assert lanes == "1" or set(got.values()) == {128}  # nothing to choose
         k.close()
+
+
+def test_closure_modes_of_a_wide_block(monkeypatch):
+    """The density kernel of each closure mode with 512 threads a block, whose shared memory passes the default limit:
+    each mode's kernel is allowed it when the mode is set."""
+    monkeypatch.setenv("SPH_GROUP_LANES", "1")
+    sc = domain.tank_with_sphere(0.004, domain_max=(0.048, 0.048, 0.06), center=(0.024, 0.024, 0.02), radius=0.01,
+                                 fill_height=0.04, hydrostatic=True, geometry="lattice")
+    out = []
+    for threads in (128, 512):
+        k = CudaKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta)
+        k.set_launch(128, threads, 128)
+        k.set_feature_sdf(sc.sdf)
+        for mode in (0, 2, 1, 0):
+            k.set_closure(mode, ClosureNet(seed=2).params() if mode == 2 else None)
+            k.step_auto(2)
+        out.append(k.particles())
+        k.close()
+    assert_same(*out)

@@ -640,31 +640,20 @@ void choose_lanes(SphHandle* h, int sms) {
   }
 }
 
-// Lets the handle's density kernels take up to 128 KiB of dynamic shared memory
-// (the warp scan's per-warp scratch passes the default 48 KiB at 512 threads)
-// on the current device. Set at handle creation, before any graph capture, and
-// only for the form in use: naming a kernel here loads it (all 18: a process's
-// first creation 34 ms, these three: 31).
-void allow_density_smem(const SphHandle* h) {
+// Lets the handle's density kernel of closure mode `mode` take up to 128 KiB of
+// dynamic shared memory (the warp scan's per-warp scratch passes the default 48
+// KiB at 512 threads) on the current device. Set at handle creation and by
+// sph_set_closure, before any graph capture, and only for the kernel that will
+// run: naming a kernel here loads it. The forms with several lanes per particle
+// stay below the default.
+void allow_density_smem(const SphHandle* h, int mode) {
   using namespace sph;
-  auto set = [](auto kernel) {
-    cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         128 * 1024);
-  };
+  if (h->lanes_density != 1) return;
   auto form = [&](auto* constants) {
     using KPT = std::remove_pointer_t<decltype(constants)>;
-    if (h->lanes_density > 2) {
-      with_lanes(h->lanes_density, [&](auto lanes) {
-        constexpr int G = decltype(lanes)::value;
-        set(k_density_group<KPT, 0, G>);
-        set(k_density_group<KPT, 1, G>);
-        set(k_density_group<KPT, 2, G>);
-      });
-    } else if (h->lanes_density == 1) {
-      set(k_density<KPT, 0>);
-      set(k_density<KPT, 1>);
-      set(k_density<KPT, 2>);
-    }
+    auto* kernel = mode == 2 ? k_density<KPT, 2> : mode == 1 ? k_density<KPT, 1> : k_density<KPT, 0>;
+    cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         128 * 1024);
   };
   if (h->ninst == 1) form(static_cast<OneSim*>(nullptr));
   else form(static_cast<ManySim*>(nullptr));
@@ -706,6 +695,7 @@ void enqueue_density_only(SphHandle* h) {
         const int grid = grid_for(h->n, kGroupThreads / G);
         constexpr size_t smem0 = (kGroupThreads / 32) * sizeof(CoopWarp<G, 2>);
         constexpr size_t smem1 = (kGroupThreads / 32) * sizeof(CoopWarp<G, 3>);
+        static_assert(smem1 + sizeof(BlockTile) <= 48 * 1024, "no attribute needed (allow_density_smem)");
         auto run = [&](auto kernel, size_t smem) {
           launch(h, kernel, grid, kGroupThreads, smem, kp, h->n, h->dt, h->pos, planes(h), h->rv, h->id, h->ctab,
                  h->bc_start, h->bc_list, h->bpos, h->rf, h->pr, h->err, h->nbr, h->ncount, h->sdf, h->wall_tab, cb,
@@ -1205,7 +1195,7 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
     int sms = 148;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->dev) != cudaSuccess) sms = 148;
     choose_lanes(h, sms);
-    allow_density_smem(h);
+    allow_density_smem(h, 0);
 #define ALLOC(ptr, cnt) \
   if (ae == cudaSuccess) ae = dalloc(h, &h->ptr, (cnt))
     ALLOC(pos, n); ALLOC(vel, n); ALLOC(velout, n); ALLOC(acc, n);
@@ -1238,6 +1228,11 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   } catch (...) {  // no thread to be had: allocate here, before the host tables
     allocate_all();
   }
+  // A process's first creation loads the kernels' module (8 ms), here beside
+  // the allocations (7 ms) instead of at its first launch.
+  cudaFuncAttributes loaded;
+  if (cudaFuncGetAttributes(&loaded, sph::k_reorder) != cudaSuccess) cudaGetLastError();
+  trace.mark("kernels loaded");
   for (int q = 0; q < ninst; ++q) {
     const SphBoundaryView* bv = (sdf_mode || !bvs) ? nullptr : bvs[q];
     h->poff[q + 1] = h->poff[q] + pvs[q].n;
@@ -2380,6 +2375,7 @@ int sph_set_closure(SphHandle* h, int mode, const float* params) {
     SPH_TRY(h, cudaMemcpyAsync(h->cl_wq, frag.data(), frag.size() * sizeof(uint32_t), cudaMemcpyHostToDevice, h->st));
     SPH_TRY(h, cudaStreamSynchronize(h->st));
   }
+  allow_density_smem(h, mode);
   h->cl_mode = mode;
   drop_graphs(h);
   return SPH_OK;
