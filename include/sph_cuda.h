@@ -28,8 +28,10 @@
  * size from which the density pass takes its warp-cooperative scan of 32
  * particles a warp (1300 particles per SM; 0 = always), and SPH_GROUP_LANES (1,
  * 8 or 16, or 2 for the density pass) sets the lanes that share a particle in
- * the neighbour kernels, which otherwise follow from the size. All forms give
- * the same results bit for bit.
+ * the neighbour kernels, which otherwise follow from the size. SPH_WALL_LISTS=0
+ * leaves out the lists of fluid particles that boundary particles keep (192
+ * bytes each); the boundary pressure then searches the grid, as it does where
+ * their memory cannot be had. All forms give the same results bit for bit.
  */
 #ifndef SPH_CUDA_H
 #define SPH_CUDA_H

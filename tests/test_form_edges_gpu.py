@@ -170,3 +170,33 @@ def test_closure_modes_of_a_wide_block(monkeypatch):
         out.append(k.particles())
         k.close()
     assert_same(*out)
+
+
+@pytest.mark.parametrize("lanes", ["1", "2", "8", "16"])
+def test_boundary_pressure_without_lists(lanes, monkeypatch):
+    """The search that stands in where the boundary particles' lists have no memory."""
+    monkeypatch.setenv("SPH_GROUP_LANES", lanes)
+    monkeypatch.setenv("SPH_WALL_LISTS", "0")
+    sc = small_dam_break()
+    gpu = CudaKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta)
+    cpu = orc.OracleKernel(*sc.kernel_args(), alpha=sc.alpha, beta=sc.beta, tier=1, threads=8, pow_mode=1)
+    for _ in range(3):
+        gpu.step(2e-5)
+        cpu.step(2e-5)
+        assert_same(gpu.particles(), cpu.particles())
+        np.testing.assert_array_equal(gpu.boundary_pressure(), cpu.boundary_pressure())
+    gpu.close()
+
+
+def test_boundary_pressure_of_a_batch_without_lists(monkeypatch):
+    scs = domain.batch_boxes(3, seed=5, dx=0.004, lo=200, hi=2000, draw="loguniform")
+    out = []
+    for lists in ("1", "0"):
+        monkeypatch.setenv("SPH_WALL_LISTS", lists)
+        b = CudaBatch(scs)
+        b.step_auto(4)
+        out.append((b.particles(), b.boundary_pressure()))
+        b.close()
+    assert_same(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
+    assert out[0][1].any()

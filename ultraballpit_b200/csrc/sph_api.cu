@@ -108,7 +108,8 @@ struct SphHandle {
   float4* bpos = nullptr;
   float* bpress = nullptr;
   // per boundary particle: the fluid particles in its support (scatter_walls;
-  // wlist null where its memory could not be had: k_adami then searches)
+  // wlist null where its memory could not be had or SPH_WALL_LISTS is 0: k_adami
+  // then searches)
   uint32_t *wcount = nullptr, *wlist = nullptr;
   int pool = -1;  // device arrays from the library's pool (1) or cudaMalloc (0); set by the first one
   // lanes per particle of the neighbour kernels (1: a thread per particle, in
@@ -1439,7 +1440,9 @@ int create_impl(int ninst, const SphParams* PP, const SphParticlesView* pvs,
   trace.mark("particle uploads joined");
   if (e == cudaSuccess) e = ue;
   if (e == cudaSuccess) e = dalloc(h, &h->bc_list, blist.size());
-  if (e == cudaSuccess && nb > 0 && dalloc(h, &h->wlist, sph::kWallCap * nb) != cudaSuccess) {
+  const char* lists = std::getenv("SPH_WALL_LISTS");
+  if (e == cudaSuccess && nb > 0 && !(lists && std::atoi(lists) == 0) &&
+      dalloc(h, &h->wlist, sph::kWallCap * nb) != cudaSuccess) {
     cudaGetLastError();
     h->wlist = nullptr;  // k_adami searches instead
   }
