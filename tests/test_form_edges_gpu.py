@@ -8,7 +8,7 @@ import pytest
 from oracle import oracle as orc
 from ultraballpit_b200 import domain
 from ultraballpit_b200.closure import ClosureNet
-from ultraballpit_b200.kernel import CudaBatch, CudaKernel
+from ultraballpit_b200.kernel import CELL_ORDER_LINEAR, CELL_ORDER_ROWS, CudaBatch, CudaKernel
 from ultraballpit_b200.particles import BoundaryParticles, ParticleArrays
 
 from test_group_forms_gpu import first
@@ -200,3 +200,34 @@ def test_boundary_pressure_of_a_batch_without_lists(monkeypatch):
     assert_same(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
     assert out[0][1].any()
+
+
+# cells of the grid: one scan kernel up to 16,384, two up to 2,097,152, three above
+@pytest.mark.parametrize("dims", [(32, 32, 16), (41, 40, 10), (128, 128, 128), (129, 128, 128), (300, 90, 90)])
+@pytest.mark.parametrize("order", [CELL_ORDER_ROWS, CELL_ORDER_LINEAR])
+def test_grids_of_many_cells(dims, order):
+    h = np.float32(1.3 * 0.004)
+    cell = np.float32(2.0) * h
+    hi = tuple(float(np.float32((d - 0.5) * cell)) for d in dims)
+    rng = np.random.default_rng(3)
+    # clumps of neighbours all over the grid, and particles in its first and last cells
+    centre = rng.uniform(0.1, 0.9, (60, 3)) * hi
+    x = (centre[:, None, :] + rng.uniform(-0.4, 0.4, (60, 10, 3)) * cell).reshape(-1, 3)
+    x[0], x[1] = 0.1 * cell, np.array(hi) - 0.1 * cell
+    p = ParticleArrays.from_positions(*x.T.astype(np.float32), 6.4e-5)
+    none = BoundaryParticles.from_arrays(*[np.zeros(0, np.float32)] * 7)
+    args = (p, none, float(h), (0.0, 0.0, -9.81), 20.0, 0.25, 0.0, (0.0, 0.0, 0.0), hi)
+    gpu = CudaKernel(*args, cell_order=order)
+    g = gpu.read_grid()
+    o = orc.grid_build(p.x, p.y, p.z, cell, args[7], args[8])
+    assert tuple(g["dims"]) == o["dims"] == dims
+    np.testing.assert_array_equal(g["cell_count"], o["counts"])
+    if order == CELL_ORDER_LINEAR:
+        np.testing.assert_array_equal(g["cell_start"], o["offsets"])
+        np.testing.assert_array_equal(g["slot_id"], o["sorted"])
+    cpu = orc.OracleKernel(*args, tier=1, threads=8, pow_mode=1)
+    for _ in range(3):
+        gpu.step(2e-5)
+        cpu.step(2e-5)
+        assert_same(gpu.particles(), cpu.particles())
+    gpu.close()
