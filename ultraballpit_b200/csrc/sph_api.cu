@@ -2301,9 +2301,7 @@ int sph_autotune(SphHandle* h, int trial_steps, SphLaunch* best) {
 static int upload_ktab(SphHandle* h) {
   h->k = h->ktab_h[0];
   drop_graphs(h);  // captured launches hold the old constants
-  if (h->ninst > 1)
-    SPH_TRY(h, cudaMemcpyAsync(h->ktab, h->ktab_h.data(), h->ninst * sizeof(SimConst), cudaMemcpyHostToDevice,
-                               h->st));
+  SPH_TRY(h, cudaMemcpyAsync(h->ktab, h->ktab_h.data(), h->ninst * sizeof(SimConst), cudaMemcpyHostToDevice, h->st));
   SPH_TRY(h, cudaStreamSynchronize(h->st));
   return SPH_OK;
 }
