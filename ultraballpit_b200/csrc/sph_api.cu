@@ -917,29 +917,49 @@ int read_dt(SphHandle* h, bool query, int count, float* dt_out) {
 // start costs more than they give. One read through the Python mirror (whose
 // arrays are backed with huge pages), before and now: 2k particles 228 -> 74
 // us, 31k 530 -> 195, 250k 2150 -> 830, 600k 4900 -> 1400, 2M 14,500 -> 3950.
-// A reader that finds the staging taken by another thread copies directly. It
-// is given back when the device's last handle is destroyed.
+//
+// Making it takes 1 to 3 ms (2 MB) or 4 to 8 (8 MB), and giving it back 0.4 or
+// 1, against some 0.05 ms a MB that it saves: a program that reads a simulation
+// once or twice never gains that. So it is made once kEnoughRead bytes have been
+// read without it, by a program that will read on. Created, read once and
+// destroyed, a simulation takes 2.2 / 8.6 / 15 / 27 ms at 2k / 31k / 250k / 838k
+// particles, where staging from the first read took 5.2 / 10.4 / 20 / 38. Until
+// then a read of up to kSmallRead comes over in pageable pieces (the driver's
+// staging; 20k particles 127 us, 31k 202, where a copy per array takes 227 and
+// 262 and the page-locked pieces 71 and 121; at 60k 428 and 353), a larger one
+// by a copy per array.
+//
+// A reader that finds it taken by another thread copies directly. It is given
+// back when the device's last handle is destroyed.
 constexpr size_t kStagePiece = 1 << 20, kStageOneThread = 8 << 20;
 constexpr unsigned kStageThreads = 4;
 constexpr size_t kStageBytes = kStageThreads * 2 * kStagePiece;
+constexpr size_t kEnoughRead = (size_t)40 << 20, kSmallRead = 2 << 20, kPageablePiece = 256 << 10;
 struct HostStage {
   std::mutex mu;
   char* p = nullptr;
   size_t bytes = 0;
   cudaStream_t st[kStageThreads] = {};
   int handles = 0;
+  size_t without = 0;  // bytes read while it was not there, or smaller than the read could use
   void give_back() {
     if (p) cudaFreeHost(p);
     p = nullptr;
-    bytes = 0;
+    bytes = without = 0;
     for (cudaStream_t& s : st) {
       if (s) cudaStreamDestroy(s);
       s = nullptr;
     }
   }
-  bool room(size_t want) {  // page-locked memory for a read of `want` bytes
+  // page-locked memory for a read of `span` bytes that can use `want`; false
+  // while there has not been enough to read
+  bool room(size_t want, size_t span) {
     want = std::min(kStageBytes, (want + 65535) / 65536 * 65536);
     if (bytes >= want) return true;
+    if (without < kEnoughRead) {
+      without += span;
+      return false;
+    }
     if (p) cudaFreeHost(p);
     p = nullptr;
     bytes = 0;
@@ -970,9 +990,33 @@ struct ReadPart {
   size_t off, bytes;  // its range of the device staging area
 };
 
+// Bytes [lo, lo + n) of the staging area, at `from`, to the parts they belong to.
+void scatter_parts(const char* from, size_t lo, size_t n, const ReadPart* parts, size_t nparts) {
+  for (size_t k = 0; k < nparts; ++k) {
+    const size_t a = std::max(lo, parts[k].off), b = std::min(lo + n, parts[k].off + parts[k].bytes);
+    if (a < b) std::memcpy((char*)parts[k].dst + (a - parts[k].off), from + (a - lo), b - a);
+  }
+}
+
 // Copies the device staging area (`span` bytes at src, ready) to the pageable
 // arrays of `parts`, and `host_bytes` of host memory beside it. False: not
 // done, the caller copies directly.
+bool read_in_pieces(SphHandle* h, const char* src, size_t span, const ReadPart* parts, size_t nparts, void* host_dst,
+                    const void* host_src, size_t host_bytes, cudaError_t* err) {
+  if (span > kSmallRead) return false;
+  const std::unique_ptr<char[]> piece(new (std::nothrow) char[std::min(span, kPageablePiece)]);
+  if (!piece) return false;
+  *err = cudaSuccess;
+  for (size_t lo = 0; lo < span && *err == cudaSuccess; lo += kPageablePiece) {
+    const size_t n = std::min(kPageablePiece, span - lo);
+    *err = cudaMemcpyAsync(piece.get(), src + lo, n, cudaMemcpyDeviceToHost, h->st);
+    if (*err == cudaSuccess) *err = cudaStreamSynchronize(h->st);
+    if (*err == cudaSuccess) scatter_parts(piece.get(), lo, n, parts, nparts);
+  }
+  if (host_bytes) std::memcpy(host_dst, host_src, host_bytes);
+  return true;
+}
+
 bool read_through_stage(SphHandle* h, const char* src, size_t span, const ReadPart* parts, size_t nparts,
                         void* host_dst, const void* host_src, size_t host_bytes, cudaError_t* err) {
   HostStage* s = host_stage(h->dev);
@@ -981,7 +1025,7 @@ bool read_through_stage(SphHandle* h, const char* src, size_t span, const ReadPa
   if (!lock.owns_lock()) return false;
   const size_t pieces = (span + kStagePiece - 1) / kStagePiece;
   const unsigned T = span <= kStageOneThread ? 1u : std::min(kStageThreads, std::max(1u, std::thread::hardware_concurrency()));
-  if (!s->room(pieces <= 1 ? span : T * 2 * kStagePiece)) return false;
+  if (!s->room(pieces <= 1 ? span : T * 2 * kStagePiece, span)) return false;
   for (unsigned t = 0; t < T; ++t)
     if (!s->st[t] && cudaStreamCreateWithFlags(&s->st[t], cudaStreamNonBlocking) != cudaSuccess) {
       cudaGetLastError();
@@ -1007,11 +1051,8 @@ bool read_through_stage(SphHandle* h, const char* src, size_t span, const ReadPa
                             cudaMemcpyDeviceToHost, s->st[t]);
       if (e != cudaSuccess) bad = (int)e;
       if (ahead < pieces && e == cudaSuccess) {
-        const size_t lo = ahead * kStagePiece, hi = std::min(span, lo + kStagePiece);
-        for (size_t k = 0; k < nparts; ++k) {
-          const size_t a = std::max(lo, parts[k].off), b = std::min(hi, parts[k].off + parts[k].bytes);
-          if (a < b) std::memcpy((char*)parts[k].dst + (a - parts[k].off), slot[w] + (a - lo), b - a);
-        }
+        const size_t lo = ahead * kStagePiece;
+        scatter_parts(slot[w], lo, std::min(kStagePiece, span - lo), parts, nparts);
       }
       if (q == pieces || e != cudaSuccess) break;
       ahead = q;
@@ -1717,8 +1758,11 @@ int sph_read_particles(SphHandle* h, SphParticlesMut* o) {
     ReadPart parts[13];
     for (int f = 0; f < 12; ++f) parts[f] = {dst[f], f * n * sizeof(float), n * sizeof(float)};
     parts[12] = {o->fluid_type, 12 * n * sizeof(float), n};
-    done = read_through_stage(h, (const char*)h->stage, n * (12 * sizeof(float) + 1), parts, o->fluid_type ? 13 : 12,
-                              o->temperature, h->temperature.data(), o->temperature ? n * sizeof(float) : 0, &e);
+    const size_t nparts = o->fluid_type ? 13 : 12, span = n * (12 * sizeof(float) + 1);
+    const size_t host = o->temperature ? n * sizeof(float) : 0;
+    const char* src = (const char*)h->stage;
+    done = read_through_stage(h, src, span, parts, nparts, o->temperature, h->temperature.data(), host, &e) ||
+           read_in_pieces(h, src, span, parts, nparts, o->temperature, h->temperature.data(), host, &e);
   }
   if (done) {
     if (e != cudaSuccess) return cuda_status(h, e, "sph_read_particles");
