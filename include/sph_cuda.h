@@ -348,7 +348,11 @@ int sph_autotune(SphHandle *h, int trial_steps, SphLaunch *best);
  * MLP 16 -> 64 -> 64 -> 4 with SiLU; BF16 operands on the tensor cores with
  * FP32 accumulation, FP32 master weights and Adam state on the device.
  * Parameters (5,508 floats): W1[64][16], b1[64], W2[64][64], b2[64],
- * W3[4][64], b3[4]. Inputs x[n][16], targets t[n][4] (host, row-major). */
+ * W3[4][64], b3[4]. Inputs x[n][16], targets t[n][4] (host, row-major).
+ * A net keeps the device buffers of its calls, up to 64 MB, for the next
+ * call; those above 1 MB come from the library's pool and go back to it with
+ * the net. Several threads may call one net: trainings and gradients follow
+ * one another, forward calls do not wait. */
 #define SPH_MLP_PARAMS 5508
 typedef struct SphMlp SphMlp;
 /* Weights and biases uniform in +-1/sqrt(fan_in) from `seed`. */

@@ -63,3 +63,25 @@ def test_forward_and_gradients_beside_training():
     np.testing.assert_array_equal(got[0], want)
     np.testing.assert_array_equal(net.params(), alone.params())
     assert any(np.array_equal(grads[0], g) for g in (before, after))
+
+
+def test_nets_that_come_and_go():
+    """Kept buffers on both sides of 1 MB and 64 MB (what comes from the library's pool), given back by one net and
+    taken by the next, and by several at a time."""
+    sizes = (500, 3000, 60000, 400000)
+    data = [_data(n, n) for n in sizes]
+    net = ClosureNet(seed=8)
+    want = [net.loss_grad(x, t) for x, t in data]
+    net.close()
+
+    def user(q):
+        def go():
+            for r in range(8):
+                i = (q + r) % len(sizes)
+                m = ClosureNet(seed=8)
+                loss, g = m.loss_grad(*data[i])
+                assert loss == want[i][0]
+                np.testing.assert_array_equal(g, want[i][1])
+                m.close()
+        return go
+    in_threads(*[user(q) for q in range(3)])

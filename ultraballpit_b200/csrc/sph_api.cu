@@ -187,12 +187,15 @@ int cuda_status(SphHandle* h, cudaError_t e, const char* what) {
     if (_e != cudaSuccess) return cuda_status(h, _e, #call); \
   } while (0)
 
+}  // namespace
+
 // The handles' device arrays come from one memory pool per device, owned by
 // this library, in stream order on the handle's stream. The pool keeps what
 // a closed handle frees (release threshold: unlimited), so a process that
 // creates simulations one after another reuses mapped memory instead of
 // asking the driver to map it again each time; the memory stays reserved for
-// this library until the process exits.
+// this library until the process exits. The closure nets' kept buffers come
+// from it too (sph_mlp.cu).
 cudaMemPool_t device_pool(int dev) {
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
@@ -210,6 +213,8 @@ cudaMemPool_t device_pool(int dev) {
   pools[dev] = pool;
   return pool;
 }
+
+namespace {
 
 template <class T>
 cudaError_t dalloc(SphHandle* h, T** p, size_t count) {
