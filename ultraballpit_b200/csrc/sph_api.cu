@@ -748,7 +748,7 @@ void enqueue_adami(SphHandle* h) {
   using namespace sph;
   if (h->nb == 0) return;
   if (h->wlist && (h->lanes_density == 1 || h->cl_mode)) {  // else the density pass has done it (scatter_walls)
-    const int P = h->n >= 1000000 ? 16 : 8;  // between 250k and 2M particles the two cross (k_wall_scatter)
+    const int P = h->n >= 1000000 ? 16 : 8;  // the table at k_wall_scatter
     dispatch(h, false, [&](auto kp) {
       launch(h, k_wall_scatter<decltype(kp)>, grid_for(h->n, 8 * P), 256, 0, kp, h->n, P, h->pos, h->nbr, h->ncount,
              h->bc_start, h->bc_list, h->bpos, wall_lists(h), h->err);
@@ -940,6 +940,7 @@ constexpr size_t kStagePiece = 1 << 20, kStageOneThread = 8 << 20;
 constexpr unsigned kStageThreads = 4;
 constexpr size_t kStageBytes = kStageThreads * 2 * kStagePiece;
 constexpr size_t kEnoughRead = (size_t)40 << 20, kSmallRead = 2 << 20, kPageablePiece = 256 << 10;
+constexpr size_t kLeastCounted = 512 << 10;  // a read counts as this at least: it saves some 10 us whatever its size
 struct HostStage {
   std::mutex mu;
   char* p = nullptr;
@@ -962,7 +963,7 @@ struct HostStage {
     want = std::min(kStageBytes, (want + 65535) / 65536 * 65536);
     if (bytes >= want) return true;
     if (without < kEnoughRead) {
-      without += span;
+      without += std::max(span, kLeastCounted);
       return false;
     }
     if (p) cudaFreeHost(p);

@@ -524,7 +524,13 @@ k_density_group(KP kp, int n, const float* __restrict__ dtp, const float4* __res
 // then the other's. It executes 38 % more instructions than 32 particles a warp
 // and halves the chain. Density, us, 8 lanes | pair | 32 particles a warp:
 //   31k 66 | 66 | 103   50k 96 | 79 | 104   73k 131 | 95 | 111
-//   146k - | 166 | 178   250k - | 251 | 241   (69k without walls - | 87 | 106)
+//   146k - | 166 | 178   250k - | 251 | 241
+// A tank with SDF walls:   24k  49 | 53 | 88     35k  66 | 55 | 88     73k 125 | 82 | 104
+//                         115k 186 | 119 | 115  163k 260 | 160 | 154  191k 301 | 174 | 162
+// and with the closure:    24k  80 | 94 | 135    35k 111 | 109 | 131   73k 195 | 152 | 164
+//                         115k 291 | 223 | 213  163k 379 | 270 | 254  191k 436 | 307 | 300
+// There two lanes and one cross at some 100k, not at the 192k that the rule has
+// for all: up to 7 % of those passes (SDF walls with the closure 14 %).
 // Eight blocks per SM at 64 registers; with six or five, 73k takes 113 or 117.
 constexpr int kPairParticles = 16;
 constexpr int kPairBlocks = 8;
