@@ -207,8 +207,8 @@ int sph_create(const SphParams *params, const SphParticlesView *particles,
  * which keeps them for the next handle created on that device (creating
  * simulations one after another then skips the driver's mapping of fresh
  * memory); the pool's memory stays reserved until the process exits. The
- * page-locked staging of reads to the host goes with the last handle that
- * counts on it. */
+ * page-locked staging (8 MB at most) that reads to the host pass through once
+ * 40 MiB have been read goes with the device's last handle. */
 void sph_destroy(SphHandle *h);
 
 /* SimulationKernel::step (lib.rs:287-335). Enqueued asynchronously. */
