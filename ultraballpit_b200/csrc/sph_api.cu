@@ -196,7 +196,8 @@ int cuda_status(SphHandle* h, cudaError_t e, const char* what) {
 // asking the driver to map it again each time; the memory stays reserved for
 // this library until the process exits. The closure nets' kept buffers come
 // from it too (sph_mlp.cu).
-cudaMemPool_t device_pool(int dev) {
+namespace sph {
+__attribute__((visibility("hidden"))) cudaMemPool_t device_pool(int dev) {
   static std::mutex mu;
   static std::map<int, cudaMemPool_t> pools;
   std::lock_guard<std::mutex> lock(mu);
@@ -213,6 +214,7 @@ cudaMemPool_t device_pool(int dev) {
   pools[dev] = pool;
   return pool;
 }
+}  // namespace sph
 
 namespace {
 
@@ -220,8 +222,8 @@ template <class T>
 cudaError_t dalloc(SphHandle* h, T** p, size_t count) {
   *p = nullptr;
   if (count == 0) count = 1;
-  if (h->pool < 0) h->pool = (h->st && device_pool(h->dev)) ? 1 : 0;  // fixed for the handle's life
-  cudaError_t e = h->pool ? cudaMallocFromPoolAsync((void**)p, count * sizeof(T), device_pool(h->dev), h->st)
+  if (h->pool < 0) h->pool = (h->st && sph::device_pool(h->dev)) ? 1 : 0;  // fixed for the handle's life
+  cudaError_t e = h->pool ? cudaMallocFromPoolAsync((void**)p, count * sizeof(T), sph::device_pool(h->dev), h->st)
                           : cudaMalloc((void**)p, count * sizeof(T));
   if (e == cudaSuccess) h->allocs.push_back((void*)*p);
   return e;

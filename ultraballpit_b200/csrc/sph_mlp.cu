@@ -20,7 +20,9 @@
 
 using namespace sphmlp;
 
-cudaMemPool_t device_pool(int dev);  // sph_api.cu: null if there is none
+namespace sph {
+__attribute__((visibility("hidden"))) cudaMemPool_t device_pool(int dev);  // sph_api.cu: null if there is none
+}
 
 struct SphMlp {
   int dev = 0;
@@ -432,7 +434,7 @@ cudaError_t ensure_work(SphMlp* h, size_t n, int rows, size_t tiles) {
   // What a net keeps comes from the library's pool: mapping 2 MB and more anew
   // takes 0.5 ms (a net created for one gradient of 2,400 samples: 1.30 ms, 0.81
   // from the pool); less than that has room in what the process has mapped.
-  const cudaMemPool_t pool = bytes > (1u << 20) && bytes <= kKeep ? device_pool(h->dev) : nullptr;
+  const cudaMemPool_t pool = bytes > (1u << 20) && bytes <= kKeep ? sph::device_pool(h->dev) : nullptr;
   h->work_pooled = pool != nullptr;
   const cudaError_t e = pool ? cudaMallocFromPoolAsync((void**)&h->work, bytes, pool, h->st)
                              : cudaMalloc((void**)&h->work, bytes);
